@@ -690,16 +690,17 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, Mi
   }
   if constexpr (MODE == 1) {
     __syncthreads();
-    if (t.partial && tid < F) {
-      // the block's L1 residual sum of field tid: cell by cell, points in
-      // order within a cell, as compute_res_upts adds them
-      double bs = 0.0;
-      for (int el = 0; el < nval; el++) {
-        double cs = 0.0;
-        for (int r = 0; r < NU; r++) cs += sRes[tid * EU + el * NU + r];
-        bs += cs;
+    if (t.partial) {
+      // the block's L1 residual sum of each field: one warp per field, lanes
+      // over the block's points and a fixed tree (one thread per field walking
+      // the points was a chain of EPB x NU dependent additions)
+      for (int k = warp; k < F; k += NW) {
+        double bs = 0.0;
+        for (int i = tid & 31; i < nuv; i += 32) bs += sRes[k * EU + i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) bs += __shfl_down_sync(0xffffffffu, bs, o);
+        if ((tid & 31) == 0) t.partial[(size_t)blockIdx.x * F + k] = bs;
       }
-      t.partial[(size_t)blockIdx.x * F + tid] = bs;
     }
     auto bu = [&](int n) { return sUn + n * Q::ldU; };
     auto one = [&](int r, int n, double v) {
