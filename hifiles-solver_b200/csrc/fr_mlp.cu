@@ -5,11 +5,13 @@
 // Training step on a batch of N samples (x_n, c*_n, weight s_n; s_n = 1 when
 // no weights are given):
 //   loss = (1/N) sum_n s_n (c(x_n) - c*_n)^2
-// fr_mlp_loss_grad_kernel: one CTA per tile of 128 samples; forward pass with
-// the activations kept in shared memory, then the backward pass as
-// tile-local sums over the samples in a fixed order -> one partial gradient
-// per CTA; fr_mlp_reduce_kernel sums the partials in CTA order, so a gradient
-// is the same bit for bit on every run.  fr_mlp_adam_kernel applies Adam.
+// fr_mlp_loss_grad_kernel: persistent CTAs, each over tiles of 128 samples
+// (tile = CTA, CTA + grid, ...); the three 64 x 64 products of a sample
+// (forward, weight gradient, input gradient) are register-tiled FP32 products
+// over shared memory, and a CTA keeps its gradient in registers over all its
+// tiles -> one partial gradient per CTA.  fr_mlp_reduce_kernel sums the
+// partials in a fixed order, so a gradient is the same bit for bit on every
+// run on one GPU model.  fr_mlp_adam_kernel applies Adam.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -25,7 +27,15 @@ extern thread_local std::string g_err;
 namespace {
 
 constexpr int kTile = 128;
-constexpr size_t kGradSmem = sizeof(float) * (kMlpIn + 2 * kMlpH + 2) * kTile;
+constexpr int kLd = kTile + 4;   // row stride of the sample-minor arrays: 8 rows at one sample fall in 8 bank groups
+// Shared memory of fr_mlp_loss_grad_kernel (floats): W2 transposed [i][j] and
+// as it is [j][i], h1 and h2 (then their loss derivatives) [unit][sample], x
+// [6][sample], partial outputs per warp [8][sample], d loss / d o [sample].
+constexpr int kGradThreads = 256, kGradWarps = kGradThreads / 32;
+constexpr int kSmW2T = 0, kSmW2 = kSmW2T + kMlpH * kMlpH, kSmH1 = kSmW2 + kMlpH * kMlpH, kSmH2 = kSmH1 + kMlpH * kLd,
+              kSmX = kSmH2 + kMlpH * kLd, kSmO = kSmX + kMlpIn * kLd, kSmDo = kSmO + kGradWarps * kTile,
+              kSmEnd = kSmDo + kTile;
+constexpr size_t kGradSmem = sizeof(float) * kSmEnd;
 
 fr_status mlp_fail(fr_status s, const std::string& m)
 {
@@ -44,116 +54,262 @@ __global__ void __launch_bounds__(256) fr_mlp_forward_kernel(const float* __rest
   out[i] = mlp_eval(w, x);
 }
 
-__global__ void __launch_bounds__(kTile) fr_mlp_loss_grad_kernel(const float* __restrict__ w,
-                                                                 const float* __restrict__ X,
-                                                                 const float* __restrict__ Y,
-                                                                 const float* __restrict__ SW, long long n,
-                                                                 float inv_n, float* __restrict__ partial)
+// acc[r][c] += w[r] v.c for 8 weights (two broadcast quads) and 4 samples
+__device__ __forceinline__ void mlp_fma_8x4(float (&acc)[8][4], const float* w8, const float* v4)
 {
-  // activations sample-minor ([unit][sample]) so that a warp's 32 samples
-  // sit in 32 banks; 68 KB of dynamic shared memory
-  extern __shared__ float mlp_smem[];
-  auto sX = reinterpret_cast<float (*)[kTile]>(mlp_smem);
-  auto sH1 = reinterpret_cast<float (*)[kTile]>(mlp_smem + kMlpIn * kTile);            // h1, then d loss / d a1
-  auto sH2 = reinterpret_cast<float (*)[kTile]>(mlp_smem + (kMlpIn + kMlpH) * kTile);  // h2, then d loss / d a2
-  float* sDo = mlp_smem + (kMlpIn + 2 * kMlpH) * kTile;
-  float* sLoss = sDo + kTile;
-  const int t = threadIdx.x;
-  const long long s = (long long)blockIdx.x * kTile + t;
-  const bool live = s < n;
-  // ---- forward, one sample per thread
-  float x[kMlpIn];
+  const float4 wa = *reinterpret_cast<const float4*>(w8), wb = *reinterpret_cast<const float4*>(w8 + 4);
+  const float4 v = *reinterpret_cast<const float4*>(v4);
+  const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
-  for (int k = 0; k < kMlpIn; k++) {
-    x[k] = live ? (X[s * kMlpIn + k] - w[kMlpXm + k]) * w[kMlpXs + k] : 0.f;
-    sX[k][t] = x[k];
-  }
-  for (int i = 0; i < kMlpH; i++) {
-    float a = w[kMlpB1 + i];
-#pragma unroll
-    for (int k = 0; k < kMlpIn; k++) a = fmaf(w[kMlpW1 + i * kMlpIn + k], x[k], a);
-    sH1[i][t] = tanhf(a);
-  }
-  float o = w[kMlpB3];
-  for (int j = 0; j < kMlpH; j++) {
-    float a = w[kMlpB2 + j];
-    for (int i = 0; i < kMlpH; i++) a = fmaf(w[kMlpW2 + j * kMlpH + i], sH1[i][t], a);
-    const float h = tanhf(a);
-    sH2[j][t] = h;
-    o = fmaf(w[kMlpW3 + j], h, o);
-  }
-  const float c = mlp_softplus(o);
-  const float r = live ? c - Y[s] : 0.f;
-  const float sw = (live && SW) ? SW[s] : 1.f;
-  const float sig = 1.f / (1.f + expf(-o));
-  sDo[t] = 2.f * sw * r * sig * inv_n;  // d loss / d o
-  sLoss[t] = sw * r * r;
-  __syncthreads();
-
-  float* P = partial + (size_t)blockIdx.x * (kMlpTrain + 1);
-  // ---- output layer: dw3_j = sum_s do h2_j, db3 = sum_s do
-  if (t < kMlpH) {
-    float acc = 0.f;
-    for (int q = 0; q < kTile; q++) acc = fmaf(sDo[q], sH2[t][q], acc);
-    P[kMlpW3 + t] = acc;
-  }
-  if (t == kMlpH) {
-    float acc = 0.f, l = 0.f;
-    for (int q = 0; q < kTile; q++) { acc += sDo[q]; l += sLoss[q]; }
-    P[kMlpB3] = acc;
-    P[kMlpTrain] = l;
-  }
-  __syncthreads();
-  // ---- d loss / d a2 = do w3_j (1 - h2_j^2), in place
-  for (int j = 0; j < kMlpH; j++) {
-    const float h = sH2[j][t];
-    sH2[j][t] = sDo[t] * w[kMlpW3 + j] * (1.f - h * h);
-  }
-  __syncthreads();
-  // ---- dW2[j][i] = sum_s da2_j h1_i, db2_j = sum_s da2_j
-  for (int e = t; e < kMlpH * kMlpH; e += kTile) {
-    const int j = e / kMlpH, i = e - j * kMlpH;
-    float acc = 0.f;
-    for (int q = 0; q < kTile; q++) acc = fmaf(sH2[j][q], sH1[i][q], acc);
-    P[kMlpW2 + e] = acc;
-  }
-  if (t < kMlpH) {
-    float acc = 0.f;
-    for (int q = 0; q < kTile; q++) acc += sH2[t][q];
-    P[kMlpB2 + t] = acc;
-  }
-  __syncthreads();
-  // ---- d loss / d a1_i = (sum_j W2[j][i] da2_j) (1 - h1_i^2), in place
-  for (int i = 0; i < kMlpH; i++) {
-    float acc = 0.f;
-    for (int j = 0; j < kMlpH; j++) acc = fmaf(w[kMlpW2 + j * kMlpH + i], sH2[j][t], acc);
-    const float h = sH1[i][t];
-    sH1[i][t] = acc * (1.f - h * h);
-  }
-  __syncthreads();
-  // ---- dW1[i][k] = sum_s da1_i x_k, db1_i = sum_s da1_i
-  for (int e = t; e < kMlpH * kMlpIn; e += kTile) {
-    const int i = e / kMlpIn, k = e - i * kMlpIn;
-    float acc = 0.f;
-    for (int q = 0; q < kTile; q++) acc = fmaf(sH1[i][q], sX[k][q], acc);
-    P[kMlpW1 + e] = acc;
-  }
-  if (t < kMlpH) {
-    float acc = 0.f;
-    for (int q = 0; q < kTile; q++) acc += sH1[t][q];
-    P[kMlpB1 + t] = acc;
+  for (int r = 0; r < 8; r++) {
+    acc[r][0] = fmaf(w[r], v.x, acc[r][0]);
+    acc[r][1] = fmaf(w[r], v.y, acc[r][1]);
+    acc[r][2] = fmaf(w[r], v.z, acc[r][2]);
+    acc[r][3] = fmaf(w[r], v.w, acc[r][3]);
   }
 }
 
-// grad[p] = sum over CTAs of partial[b][p] (CTA order); loss = sum of the
-// per-CTA squared residuals / n.
-__global__ void fr_mlp_reduce_kernel(const float* __restrict__ partial, int nblk, float inv_n,
-                                     float* __restrict__ grad, float* __restrict__ loss)
+// Bound: FP32 FMA issue, 13.6 k multiply-adds a sample (24 us of FP32 peak for
+// 65536 samples).  A product over [unit][sample] arrays gives each warp 8
+// units and all 128 samples, 4 per lane: 8 x 4 register tile, so 3 16-byte
+// shared loads (2 of them broadcasts) feed 32 FMAs; the weight gradient takes
+// a 4 x 4 tile per thread with K = the samples, 8 loads per 64 FMAs.  Both
+// leave the FMA pipe ahead of the shared-memory pipe; one output per thread
+// with two loads per FMA was bound by the latter, and left 512 partials to add
+// (a step with its reduction and Adam, 65536 samples: 240 us, now 76).
+__global__ void __launch_bounds__(kGradThreads, 2) fr_mlp_loss_grad_kernel(const float* __restrict__ w,
+                                                                           const float* __restrict__ X,
+                                                                           const float* __restrict__ Y,
+                                                                           const float* __restrict__ SW, long long n,
+                                                                           float inv_n, float* __restrict__ partial)
 {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p > kMlpTrain) return;
+  extern __shared__ __align__(16) float mlp_smem[];
+  float* sW2T = mlp_smem + kSmW2T;
+  float* sW2 = mlp_smem + kSmW2;
+  float* sH1 = mlp_smem + kSmH1;   // h1, then d loss / d a1
+  float* sH2 = mlp_smem + kSmH2;   // d loss / d a2
+  float* sX = mlp_smem + kSmX;
+  float* sO = mlp_smem + kSmO;
+  float* sDo = mlp_smem + kSmDo;
+  const int t = threadIdx.x, lane = t & 31, wp = t >> 5, s4 = 4 * lane, u0 = 8 * wp;
+  for (int e = t; e < kMlpH * kMlpH; e += kGradThreads) {
+    const float v = w[kMlpW2 + e];
+    sW2[e] = v;
+    sW2T[(e % kMlpH) * kMlpH + e / kMlpH] = v;
+  }
+  // weight-gradient tile: rows j0 + 8 q of d a2, rows i0 + 4 p of h1
+  const int j0 = (lane & 7) + 32 * (wp & 1), i0 = (lane >> 3) + 16 * (wp >> 1);
+  // first-layer gradient: unit t / 4, quarter t % 4 of the samples
+  const int iu = t >> 2, qu = t & 3;
+  float gW2[4][4], gW1[kMlpIn], gB1 = 0.f, gW3[8], gB2[8], gB3 = 0.f, gL = 0.f;
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int p = 0; p < 4; p++) gW2[q][p] = 0.f;
+#pragma unroll
+  for (int k = 0; k < kMlpIn; k++) gW1[k] = 0.f;
+#pragma unroll
+  for (int r = 0; r < 8; r++) gW3[r] = gB2[r] = 0.f;
+
+  const long long ntile = (n + kTile - 1) / kTile;
+  for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+    const long long b0 = tile * kTile;
+    const int live = (int)(n - b0 < kTile ? n - b0 : kTile);
+    __syncthreads();   // the tile before has been read
+    for (int e = t; e < kMlpIn * kTile; e += kGradThreads) {
+      const int sm = e / kMlpIn, k = e - sm * kMlpIn;
+      sX[k * kLd + sm] = sm < live ? (X[b0 * kMlpIn + e] - w[kMlpXm + k]) * w[kMlpXs + k] : 0.f;
+    }
+    __syncthreads();
+    // ---- layer 1: units u0 .. u0 + 7, samples s4 .. s4 + 3
+    {
+      float4 x[kMlpIn];
+#pragma unroll
+      for (int k = 0; k < kMlpIn; k++) x[k] = *reinterpret_cast<const float4*>(sX + k * kLd + s4);
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const float b = __ldg(w + kMlpB1 + u0 + r);
+        float4 a = make_float4(b, b, b, b);
+#pragma unroll
+        for (int k = 0; k < kMlpIn; k++) {
+          const float c = __ldg(w + kMlpW1 + (u0 + r) * kMlpIn + k);
+          a.x = fmaf(c, x[k].x, a.x);
+          a.y = fmaf(c, x[k].y, a.y);
+          a.z = fmaf(c, x[k].z, a.z);
+          a.w = fmaf(c, x[k].w, a.w);
+        }
+        *reinterpret_cast<float4*>(sH1 + (u0 + r) * kLd + s4) =
+            make_float4(tanhf(a.x), tanhf(a.y), tanhf(a.z), tanhf(a.w));
+      }
+    }
+    __syncthreads();
+    // ---- layer 2 and this warp's share of the output
+    float h2[8][4];
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) h2[r][c] = __ldg(w + kMlpB2 + u0 + r);
+#pragma unroll 4
+    for (int i = 0; i < kMlpH; i++) mlp_fma_8x4(h2, sW2T + i * kMlpH + u0, sH1 + i * kLd + s4);
+    {
+      float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const float w3 = __ldg(w + kMlpW3 + u0 + r);
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          h2[r][c] = tanhf(h2[r][c]);
+          o[c] = fmaf(w3, h2[r][c], o[c]);
+        }
+      }
+      *reinterpret_cast<float4*>(sO + wp * kTile + s4) = make_float4(o[0], o[1], o[2], o[3]);
+    }
+    __syncthreads();
+    if (t < kTile) {
+      float o = w[kMlpB3];
+#pragma unroll
+      for (int q = 0; q < kGradWarps; q++) o += sO[q * kTile + t];
+      const bool lv = t < live;
+      const float r = lv ? mlp_softplus(o) - Y[b0 + t] : 0.f;
+      const float sw = (lv && SW) ? SW[b0 + t] : 1.f;
+      const float sig = 1.f / (1.f + expf(-o));
+      const float d = 2.f * sw * r * sig * inv_n;   // d loss / d o
+      sDo[t] = d;
+      gB3 += d;
+      gL = fmaf(sw * r, r, gL);
+    }
+    __syncthreads();
+    // ---- output layer's gradient and d loss / d a2 = do w3_j (1 - h2_j^2)
+    {
+      const float4 d4 = *reinterpret_cast<const float4*>(sDo + s4);
+      const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const float w3 = __ldg(w + kMlpW3 + u0 + r);
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          const float h = h2[r][c];
+          gW3[r] = fmaf(d[c], h, gW3[r]);
+          h2[r][c] = d[c] * w3 * (1.f - h * h);
+          gB2[r] += h2[r][c];
+        }
+        *reinterpret_cast<float4*>(sH2 + (u0 + r) * kLd + s4) = make_float4(h2[r][0], h2[r][1], h2[r][2], h2[r][3]);
+      }
+    }
+    __syncthreads();
+    // ---- dW2[j][i] += sum_s da2_j h1_i
+#pragma unroll 2
+    for (int s = 0; s < kTile; s += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) a[q] = *reinterpret_cast<const float4*>(sH2 + (j0 + 8 * q) * kLd + s);
+#pragma unroll
+      for (int p = 0; p < 4; p++) b[p] = *reinterpret_cast<const float4*>(sH1 + (i0 + 4 * p) * kLd + s);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+          gW2[q][p] = fmaf(a[q].w, b[p].w, fmaf(a[q].z, b[p].z, fmaf(a[q].y, b[p].y, fmaf(a[q].x, b[p].x, gW2[q][p]))));
+    }
+    // ---- d loss / d a1_i = (sum_j W2[j][i] da2_j) (1 - h1_i^2), in place
+    float da[8][4];
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) da[r][c] = 0.f;
+#pragma unroll 4
+    for (int j = 0; j < kMlpH; j++) mlp_fma_8x4(da, sW2 + j * kMlpH + u0, sH2 + j * kLd + s4);
+    __syncthreads();   // every thread has read h1 for dW2
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      float4* q = reinterpret_cast<float4*>(sH1 + (u0 + r) * kLd + s4);
+      const float4 h = *q;
+      *q = make_float4(da[r][0] * (1.f - h.x * h.x), da[r][1] * (1.f - h.y * h.y), da[r][2] * (1.f - h.z * h.z),
+                       da[r][3] * (1.f - h.w * h.w));
+    }
+    __syncthreads();
+    // ---- dW1[i][k] += sum_s da1_i x_k, db1_i += sum_s da1_i over a quarter of the samples
+#pragma unroll 2
+    for (int s = 4 * qu; s < kTile; s += 16) {
+      const float4 a = *reinterpret_cast<const float4*>(sH1 + iu * kLd + s);
+      gB1 += (a.x + a.y) + (a.z + a.w);
+#pragma unroll
+      for (int k = 0; k < kMlpIn; k++) {
+        const float4 x = *reinterpret_cast<const float4*>(sX + k * kLd + s);
+        gW1[k] = fmaf(a.w, x.w, fmaf(a.z, x.z, fmaf(a.y, x.y, fmaf(a.x, x.x, gW1[k]))));
+      }
+    }
+  }
+  // ---- this CTA's partial gradient and loss
+  float* P = partial + (size_t)blockIdx.x * (kMlpTrain + 1);
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int p = 0; p < 4; p++) P[kMlpW2 + (j0 + 8 * q) * kMlpH + i0 + 4 * p] = gW2[q][p];
+#pragma unroll
+  for (int k = 0; k < kMlpIn; k++) {
+    gW1[k] += __shfl_xor_sync(0xffffffffu, gW1[k], 1);
+    gW1[k] += __shfl_xor_sync(0xffffffffu, gW1[k], 2);
+    if (qu == 0) P[kMlpW1 + iu * kMlpIn + k] = gW1[k];
+  }
+  gB1 += __shfl_xor_sync(0xffffffffu, gB1, 1);
+  gB1 += __shfl_xor_sync(0xffffffffu, gB1, 2);
+  if (qu == 0) P[kMlpB1 + iu] = gB1;
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      gW3[r] += __shfl_xor_sync(0xffffffffu, gW3[r], o);
+      gB2[r] += __shfl_xor_sync(0xffffffffu, gB2[r], o);
+    }
+    if (lane == 0) {
+      P[kMlpW3 + u0 + r] = gW3[r];
+      P[kMlpB2 + u0 + r] = gB2[r];
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    gB3 += __shfl_xor_sync(0xffffffffu, gB3, o);
+    gL += __shfl_xor_sync(0xffffffffu, gL, o);
+  }
+  __syncthreads();
+  if (lane == 0) {   // zero in the warps without samples of their own
+    sO[wp] = gB3;
+    sO[kGradWarps + wp] = gL;
+  }
+  __syncthreads();
+  if (t == 0) {
+    float b3 = 0.f, l = 0.f;
+    for (int q = 0; q < kGradWarps; q++) {
+      b3 += sO[q];
+      l += sO[kGradWarps + q];
+    }
+    P[kMlpB3] = b3;
+    P[kMlpTrain] = l;
+  }
+}
+
+// grad[p] = sum over CTAs of partial[b][p]; loss = sum of the per-CTA squared
+// residuals / n.  A block takes 32 parameters: 8 rows of threads over the
+// partials (coalesced 128-byte reads), then the rows in order.
+constexpr int kRedRows = 8;
+__global__ void __launch_bounds__(32 * kRedRows) fr_mlp_reduce_kernel(const float* __restrict__ partial, int nblk,
+                                                                      float inv_n, float* __restrict__ grad,
+                                                                      float* __restrict__ loss)
+{
+  __shared__ float s[kRedRows][32];
+  const int c = threadIdx.x & 31, r = threadIdx.x >> 5, p = blockIdx.x * 32 + c;
   float acc = 0.f;
-  for (int b = 0; b < nblk; b++) acc += partial[(size_t)b * (kMlpTrain + 1) + p];
+  if (p <= kMlpTrain) {
+#pragma unroll 4
+    for (int b = r; b < nblk; b += kRedRows) acc += partial[(size_t)b * (kMlpTrain + 1) + p];
+  }
+  s[r][c] = acc;
+  __syncthreads();
+  if (r > 0 || p > kMlpTrain) return;
+  acc = 0.f;
+#pragma unroll
+  for (int q = 0; q < kRedRows; q++) acc += s[q][c];
   if (p < kMlpTrain) grad[p] = acc;
   else if (loss) *loss = acc * inv_n;
 }
@@ -257,8 +413,14 @@ fr_status fr_mlp_loss_grad(const float* w, const float* x, const float* y, const
   static bool once = (cudaFuncSetAttribute(fr_mlp_loss_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)kGradSmem), true);
   (void)once;
-  fr_mlp_loss_grad_kernel<<<(unsigned)nblk, kTile, kGradSmem, st>>>(w, x, y, sw, n, inv_n, scratch);
-  fr_mlp_reduce_kernel<<<(kMlpTrain + 1 + 255) / 256, 256, 0, st>>>(scratch, (int)nblk, inv_n, grad, loss);
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+    return mlp_fail(FR_ERR_CUDA, "device query failed");
+  // two CTAs per SM (104 KB of shared memory each), at most one per tile
+  const int grid = (int)(nblk < 2LL * sms ? nblk : 2LL * sms);
+  fr_mlp_loss_grad_kernel<<<grid, kGradThreads, kGradSmem, st>>>(w, x, y, sw, n, inv_n, scratch);
+  fr_mlp_reduce_kernel<<<(kMlpTrain + 1 + 31) / 32, 32 * kRedRows, 0, st>>>(scratch, grid, inv_n, grad, loss);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? FR_OK : mlp_fail(FR_ERR_CUDA, cudaGetErrorString(e));
 }
