@@ -18,8 +18,8 @@ namespace frb {
 
 thread_local std::string g_err;
 
-// blocks of the integral-diagnostics kernel (partial sums added in block order)
-constexpr int kDiagBlocks = 296;
+// most blocks of the integral-diagnostics kernel (five of 128 threads per SM)
+constexpr int kDiagBlocks = 740;
 
 cudaError_t launch_sgs_inputs(int dims, int tc_size, const double* U, const void* G, const double* detj, long long npts,
                               int nu, long long E, int order, double filter_ratio, float* X, cudaStream_t st);
