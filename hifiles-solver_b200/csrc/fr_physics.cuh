@@ -30,6 +30,7 @@ struct Phys {
 template <typename T>
 struct PhysT {
   T gamma, gm1, prandtl, mu_inf, rt_inf, c_sth, fix_vis, tau, pen_fact, filter_ratio;
+  T kg_inf;   // mu_inf / prandtl * gamma: the heat-flux factor of a fixed viscosity
   int sgs_model;
   const float* mlp;
   T bdy[14], R_ref;
@@ -39,6 +40,7 @@ struct PhysT {
     q.rt_inf = (T)p.rt_inf; q.c_sth = (T)p.c_sth; q.fix_vis = (T)p.fix_vis; q.tau = (T)p.tau;
     q.pen_fact = (T)p.pen_fact; q.filter_ratio = (T)p.filter_ratio; q.sgs_model = p.sgs_model;
     q.mlp = p.mlp;
+    q.kg_inf = q.mu_inf / q.prandtl * q.gamma;
     for (int i = 0; i < 14; i++) q.bdy[i] = (T)p.bdy[i];
     q.R_ref = (T)p.R_ref;
     return q;
@@ -55,19 +57,43 @@ template <typename T> __device__ __forceinline__ T fr_pow15(T x);
 template <> __device__ __forceinline__ double fr_pow15<double>(double x) { return pow(x, 1.5); }
 template <> __device__ __forceinline__ float fr_pow15<float>(float x) { return powf(x, 1.5f); }
 
-// Inviscid flux f[k][l] (field k, direction l): calc_invf_2d / calc_invf_3d,
-// src/flux.cpp:36-128.
-template <int D, typename T>
-__device__ __forceinline__ void inv_flux(const PhysT<T>& ph, const T* u, T (*f)[D])
+__device__ __forceinline__ double fr_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fr_fma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fr_rcp(double x) { return __drcp_rn(x); }
+__device__ __forceinline__ float fr_rcp(float x) { return __frcp_rn(x); }
+
+// a / b from r = 1 / b (rounded to nearest): the product and one correction by
+// its exact remainder, which rounds like the division itself (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990) for normal a, b and quotient.  Several quotients by one denominator
+// then cost one reciprocal and three instructions each; the D velocities of a
+// state were D divisions of 20-odd instructions.
+template <typename T>
+__device__ __forceinline__ T fr_quot(T a, T b, T r)
 {
-  constexpr int F = D + 2;
-  T v[D];
+  const T q = a * r;
+  return fr_fma(fr_fma(-q, b, a), r, q);
+}
+
+// Velocity and pressure of a state, as calc_invf_2d / calc_invf_3d form them.
+template <int D, typename T>
+__device__ __forceinline__ void inv_state(const PhysT<T>& ph, const T* u, T* v, T& p)
+{
+  const T r = fr_rcp(u[0]);
 #pragma unroll
-  for (int l = 0; l < D; l++) v[l] = u[l + 1] / u[0];
+  for (int l = 0; l < D; l++) v[l] = fr_quot<T>(u[l + 1], u[0], r);
   T ke = v[0] * v[0];
 #pragma unroll
   for (int l = 1; l < D; l++) ke = ke + v[l] * v[l];
-  T p = ph.gm1 * (u[F - 1] - (T(0.5) * u[0] * ke));
+  p = ph.gm1 * (u[D + 1] - (T(0.5) * u[0] * ke));
+}
+
+// Inviscid flux f[k][l] (field k, direction l): calc_invf_2d / calc_invf_3d,
+// src/flux.cpp:36-128, from the velocity and pressure of inv_state.
+template <int D, typename T>
+__device__ __forceinline__ void inv_flux_vp(const T* u, const T* v, T p, T (*f)[D])
+{
+  constexpr int F = D + 2;
 #pragma unroll
   for (int l = 0; l < D; l++) {
     f[0][l] = u[l + 1];
@@ -75,6 +101,13 @@ __device__ __forceinline__ void inv_flux(const PhysT<T>& ph, const T* u, T (*f)[
     for (int m = 0; m < D; m++) f[m + 1][l] = (m == l) ? p + (u[m + 1] * v[l]) : u[m + 1] * v[l];
     f[F - 1][l] = v[l] * (u[F - 1] + p);
   }
+}
+template <int D, typename T>
+__device__ __forceinline__ void inv_flux(const PhysT<T>& ph, const T* u, T (*f)[D])
+{
+  T v[D], p;
+  inv_state<D, T>(ph, u, v, p);
+  inv_flux_vp<D, T>(u, v, p, f);
 }
 
 // Viscous flux, no turbulence model: calc_visf_2d / calc_visf_3d,
@@ -143,8 +176,6 @@ __device__ __forceinline__ void vis_flux(const PhysT<T>& ph, const T* u, T (*g)[
 // where the result only enters through the viscous terms, whose size is
 // ~1/Re of the inviscid flux they are added to: its ulp-level differences from
 // the reference's division form stay far below the rounding of the total flux.
-__device__ __forceinline__ double fr_fma(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float fr_fma(float a, float b, float c) { return fmaf(a, b, c); }
 
 // Shared part of the viscous flux: velocity v, stress tau and the heat-flux
 // term q[l] = (mu gamma / Pr) de/dx_l of calc_visf_3d (src/flux.cpp:263-431).
@@ -153,20 +184,22 @@ __device__ __forceinline__ void vis_core(const PhysT<T>& ph, const T* u, T (*g)[
                                          T (&q)[D])
 {
   constexpr int F = D + 2;
-  const T rho = u[0], ri = T(1) / rho;
+  const T rho = u[0], ri = fr_rcp(rho);
 #pragma unroll
   for (int l = 0; l < D; l++) v[l] = u[l + 1] * ri;
   T ke = v[0] * v[0];
 #pragma unroll
   for (int l = 1; l < D; l++) ke = fr_fma(v[l], v[l], ke);
   T inte = fr_fma(T(-0.5), ke, u[F - 1] * ri);
-  T mu;
+  T mu, kg;
   if (ph.fix_vis == T(1)) {
     mu = ph.mu_inf;
+    kg = ph.kg_inf;
   } else {
     T rt = ph.gm1 * inte / ph.rt_inf;
     mu = ph.mu_inf * fr_pow15<T>(rt) * (T(1) + ph.c_sth) / (rt + ph.c_sth);
     mu = mu + ph.fix_vis * (ph.mu_inf - mu);
+    kg = mu / ph.prandtl * ph.gamma;
   }
   T dv[D][D];
 #pragma unroll
@@ -186,7 +219,7 @@ __device__ __forceinline__ void vis_core(const PhysT<T>& ph, const T* u, T (*g)[
 #pragma unroll
   for (int l = 1; l < D; l++) dsum = dsum + dv[l][l];
   const T diag = dsum * T(1.0 / 3.0);
-  const T kg = mu / ph.prandtl * ph.gamma, mu2 = T(2) * mu;
+  const T mu2 = T(2) * mu;
 #pragma unroll
   for (int m = 0; m < D; m++)
 #pragma unroll
@@ -237,26 +270,25 @@ __device__ __forceinline__ void vis_flux_proj(const PhysT<T>& ph, const T* u, T 
 }
 
 // Rusanov common normal flux, static mesh: inters::rusanov_flux,
-// src/inters.cpp:311-365 (the grid-velocity term v_g . n is zero).
+// src/inters.cpp:311-365 (the grid-velocity term v_g . n is zero).  The
+// reference's sqrt(0.25 s s), s = vn_l + vn_r, is |s| / 2: the square root of
+// a rounded square returns its argument in binary arithmetic.
 template <int D, typename T>
 __device__ __forceinline__ void rusanov(const PhysT<T>& ph, const T* ul, const T* ur, const T* n, T* fn)
 {
   constexpr int F = D + 2;
+  T vl[D], vr[D], pl, pr;
+  inv_state<D, T>(ph, ul, vl, pl);
+  inv_state<D, T>(ph, ur, vr, pr);
   T fl[F][D], fr[F][D];
-  inv_flux<D, T>(ph, ul, fl);
-  inv_flux<D, T>(ph, ur, fr);
-  T vl[D], vr[D];
-#pragma unroll
-  for (int l = 0; l < D; l++) { vl[l] = ul[l + 1] / ul[0]; vr[l] = ur[l + 1] / ur[0]; }
-  T vnl = vl[0] * n[0], vnr = vr[0] * n[0], kl = vl[0] * vl[0], kr = vr[0] * vr[0];
+  inv_flux_vp<D, T>(ul, vl, pl, fl);
+  inv_flux_vp<D, T>(ur, vr, pr, fr);
+  T vnl = vl[0] * n[0], vnr = vr[0] * n[0];
 #pragma unroll
   for (int l = 1; l < D; l++) {
     vnl = vnl + vl[l] * n[l]; vnr = vnr + vr[l] * n[l];
-    kl = kl + vl[l] * vl[l]; kr = kr + vr[l] * vr[l];
   }
-  T pl = ph.gm1 * (ul[F - 1] - (T(0.5) * ul[0] * kl));
-  T pr = ph.gm1 * (ur[F - 1] - (T(0.5) * ur[0] * kr));
-  T vav = fr_sqrt<T>(T(0.25) * (vnl + vnr) * (vnl + vnr));
+  T vav = fr_abs<T>(T(0.5) * (vnl + vnr));
   T cav = fr_sqrt<T>((ph.gamma * (pl + pr)) / (ul[0] + ur[0]));
   T eig = fr_abs<T>(vav + cav);
 #pragma unroll
