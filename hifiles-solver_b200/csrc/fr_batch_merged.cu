@@ -15,44 +15,35 @@ namespace {
 template <int P, typename TC>
 constexpr size_t merged_grad_smem()
 {
-  constexpr int EPB = MergedTile<P>::epb;
-  return grad_smem_bytes<3, P, EPB, TC, 0, grad_alias<3, P, EPB, kMergedNT, TC, 0, 0>()>();
+  return grad_smem_bytes<3, P, MergedTile<P>::epb, TC>();
 }
 
 template <int P, typename TC>
 constexpr size_t merged_upd_smem()
 {
-  constexpr int EPB = MergedTile<P>::epb;
-  if constexpr (merged_fused<P, TC>()) return face_update_smem_bytes<3, P, TC, 1, 1, EPB, kMergedNT>();
-  else return update_smem_bytes<3, P, EPB, kMergedNT, 1, 1, TC>();
+  return update_smem_bytes<3, P, MergedTile<P>::epb, kMergedNT, 1, 1, TC>();
 }
 
 template <int P, typename TC>
 __device__ __forceinline__ void grad_slot(const MergedGrad<TC>& g, long long b)
 {
-  fr_grad_body<3, P, MergedTile<P>::epb, kMergedNT, TC, 0, 1, 0>(b, 0, g.U, g.UF, g.mate, g.side, g.JG, g.detj, g.nL,
-                                                                 g.VF, g.ND, g.DV, g.E, g.L, g.ph, nullptr, g.BV);
+  fr_grad_body<3, P, MergedTile<P>::epb, kMergedNT, TC>(b, 0, g.U, g.UF, g.mate, g.side, g.JG, g.detj, g.nL, g.VF,
+                                                             g.ND, g.DV, g.E, g.L, g.ph, nullptr, g.BV);
 }
 
 template <int P, typename TC>
 __device__ __forceinline__ void upd_slot(const MergedUpd<TC>& u, long long b)
 {
-  constexpr int EPB = MergedTile<P>::epb;
-  if constexpr (merged_fused<P, TC>())
-    fr_face_update_body<3, P, EPB, kMergedNT, 1, 1, TC, 0>(b, u.U, u.REG, u.UFn, u.UF, u.mate, u.side, u.VF, u.ND,
-                                                           u.DV, u.JG, u.nL, u.tdA, u.idetj, u.BV, u.DIV, nullptr,
-                                                           u.E, u.L, u.ph, u.rk_a, u.rk_b, u.dt, u.first_stage,
-                                                           u.err);
-  else
-    fr_update_body<3, P, EPB, kMergedNT, 1, 1, TC>(b, u.U, u.REG, u.UFn, u.CF, u.ND, u.DV, u.JG, u.detj64, u.DIV,
-                                                   nullptr, u.E, u.L, u.ph, u.rk_a, u.rk_b, u.dt, u.first_stage);
+  fr_update_body<3, P, MergedTile<P>::epb, kMergedNT, 1, 1, TC, update_fused<3, P>() ? 1 : 0>(
+      b, u.U, u.REG, u.UFn, u.UF, u.CF, u.mate, u.side, u.VF, u.ND, u.DV, u.JG, u.nL, u.tdA, u.idetj, u.BV, u.DIV,
+      nullptr, u.E, u.L, u.ph, u.rk_a, u.rk_b, u.dt, u.first_stage);
 }
 
 template <typename TC, int MINB>
 __global__ void __launch_bounds__(kMergedNT, MINB) fr_merged_grad_kernel(const __grid_constant__ MergedGrads<TC> a)
 {
   long long b = blockIdx.x;
-  if (b < a.s[0].nblk) { grad_slot<2>(a.s[0], b); return; }
+  if (b < a.s[0].nblk) { grad_slot<2, TC>(a.s[0], b); return; }
   b -= a.s[0].nblk;
   if (b < a.s[1].nblk) { grad_slot<3>(a.s[1], b); return; }
   b -= a.s[1].nblk;

@@ -8,21 +8,21 @@
 // 2, 3 and 4: the grid is the concatenation of the groups' element blocks,
 // and each block runs the body of its group's order on that group's buffers
 // (one body per block, chosen by the block index, so every barrier of a body
-// is reached by the whole block).  All groups use 128-thread tiles (order 2:
-// 4 elements per block, order 3: 2, order 4: 1); order 3 takes the fused
-// interface/update body, orders 2 and 4 the interface-flux and update
-// bodies.  No norms are formed (the batch reports none).
+// is reached by the whole block).  All groups use blocks of 192 threads with
+// as many elements as give each flux point a thread; order 3 takes the fused interface/update body, orders 2 and 4
+// the interface-flux and update bodies.  No norms are formed (the batch reports
+// none).
 #pragma once
 
 #include "fr_b200.h"
-#include "fr_face_update.cuh"
+#include "fr_update.cuh"
 
 namespace frb {
 
-constexpr int kMergedNT = 128;
-template <int P> struct MergedTile { static constexpr int epb = P == 2 ? 4 : P == 3 ? 2 : 1; };
-// orders whose stage takes the fused interface/update kernel
-template <int P, typename TC> __host__ __device__ constexpr bool merged_fused() { return fu_bulk_ok<3, P, TC>(); }
+// threads per block and elements per block: 162, 192 and 150 of 192 threads
+// have a flux point
+constexpr int kMergedNT = 192;
+template <int P> struct MergedTile { static constexpr int epb = P == 2 ? 3 : P == 3 ? 2 : 1; };
 
 template <typename TC>
 struct MergedGrad {
@@ -44,8 +44,8 @@ struct MergedFace {
 template <typename TC>
 struct MergedUpd {
   double* U; double* REG; TC* UFn; const TC* UF; const TC* CF; const int* mate; const unsigned char* side;
-  const TC* VF; const TC* ND; const TC* DV; const TC* JG; const TC* nL; const TC* tdA; const double* detj64;
-  const double* idetj; const TC* BV; double* DIV; int* err;
+  const TC* VF; const TC* ND; const TC* DV; const TC* JG; const TC* nL; const TC* tdA;
+  const double* idetj; const TC* BV; double* DIV;
   long long E, nblk;
   Line<TC> L;
   PhysT<TC> ph;

@@ -3,11 +3,12 @@
 //
 // One RK stage of the reference (CalcResidual, src/solver.cpp:65-225, then
 // eles::AdvanceSolution, src/eles.cpp:1091-1188) runs as
-//   viscous :  fr_grad_kernel -> fr_face_kernel -> fr_update_kernel
-//   inviscid:                    fr_face_kernel -> fr_update_kernel
-// The element kernels are element-blocked: a CTA owns EPB elements, stages their solution in
-// shared memory, and applies the reference's operators as 1-D line
-// contractions (every dense operator opp_0..opp_6 of a Gauss-point tensor
+//   viscous :  fr_grad_kernel -> [fr_face_kernel ->] fr_update_kernel
+//   inviscid:                    [fr_face_kernel ->] fr_update_kernel
+// with the interface kernel folded into the update where that is the faster
+// form (fr_update.cuh).  The element kernels are element-blocked: a CTA owns
+// EPB elements, stages their solution in shared memory, and applies the
+// reference's operators as 1-D line contractions (every dense operator opp_0..opp_6 of a Gauss-point tensor
 // element has exactly one non-trivial factor per line, so the contraction
 // reproduces the dense product term by term).  Elements exchange data only
 // through flux-point traces in HBM:
@@ -144,73 +145,41 @@ __device__ __forceinline__ int upt_stride(int axis)
   return axis == 0 ? 1 : (axis == 1 ? N1 : N1 * N1);
 }
 
-// Sum over all axes of the 1-D derivative along each axis of a field stored
-// point-major: the reference's sum_d opp_2[d] (or opp_4[d]) row of u, in
-// column order per axis and axes in order.
-template <int DIM, int P, typename T, typename S>
-__device__ __forceinline__ T deriv_line(const Line<T>& L, const S* s, int sst, int u, int d, int i)
+// Faces at the two ends of the lines along axis d (minus end, plus end).
+template <int DIM>
+__host__ __device__ constexpr int line_face(int d, int plus)
 {
-  const int st = upt_stride<DIM, P>(d), ub = u - i * st;
-  T acc = T(0);
-#pragma unroll
-  for (int m = 0; m <= P; m++) acc = acc + (T)s[(ub + m * st) * sst] * L.D[i][m];
-  return acc;
+  return DIM == 2 ? (d == 0 ? (plus ? 1 : 3) : (plus ? 2 : 0))
+                  : (d == 0 ? (plus ? 2 : 4) : (d == 1 ? (plus ? 3 : 1) : (plus ? 5 : 0)));
 }
 
-// Per-block copy of the operator pieces that threads index with their own
-// (divergent) point indices, plus a table with the line of every flux point:
-// code = u0 | stride << 8 | axis << 16 | plus << 18.  Reading these from
-// shared memory avoids both serialised constant-bank loads and divergent
-// branches on the face index.
-template <typename T, int NF>
-struct BlockOps {
-  T D[kMaxN1][kMaxN1];
-  T gL[kMaxN1], gR[kMaxN1];
-  int code[NF];
-};
-
-template <typename T, int NF>
-__host__ __device__ constexpr size_t blockops_bytes()
-{
-  return (sizeof(BlockOps<T, NF>) + 15) / 16 * 16;
-}
-
-template <int DIM, int P, typename T, int NF>
-__device__ __forceinline__ void fill_blockops(BlockOps<T, NF>* B, const Line<T>& L, int tid, int nt)
-{
-  for (int i = tid; i < kMaxN1 * kMaxN1; i += nt) B->D[i / kMaxN1][i % kMaxN1] = L.D[i / kMaxN1][i % kMaxN1];
-  for (int i = tid; i < kMaxN1; i += nt) { B->gL[i] = L.gL[i]; B->gR[i] = L.gR[i]; }
-  for (int f = tid; f < NF; f += nt) {
-    int u0, st, ax; bool plus;
-    fpt_line<DIM, P>(f, u0, st, ax, plus);
-    B->code[f] = u0 | (st << 8) | (ax << 16) | ((plus ? 1 : 0) << 18);
+// Shared-memory order of a field's solution points: point (a, b, c) of an
+// element at a + S1 b + S2 c, N words per element.  Hexahedra of P = 3 pad
+// the z-planes of 16 points (18 doubles, 20 floats): lines along x are then
+// read as whole 16-byte vectors without bank conflicts, lines along z too,
+// lines along y with 2-way conflicts in FP64 and none in FP32 (unpadded: 4-way
+// along y).  The other point counts are free of conflicts, or 2-way, as they are.
+template <int DIM, int P, typename TC>
+struct PtMap {
+  static constexpr int N1 = P + 1;
+  static constexpr int S1 = N1;
+  static constexpr int S2 = DIM == 3 ? (N1 == 4 ? (sizeof(TC) == 8 ? 18 : 20) : N1 * N1) : 0;
+  static constexpr int N = DIM == 3 ? S2 * N1 : N1 * N1;
+  static constexpr int PLANE = DIM == 3 ? N1 * N1 : N1 * N1;   // points per unpadded run
+  __device__ static __forceinline__ int slot(int a, int b, int c) { return a + S1 * b + S2 * c; }
+  __host__ __device__ static constexpr int stride(int d) { return d == 0 ? 1 : (d == 1 ? S1 : S2); }
+  // slot of the first point of line (j0, j1) along axis d, whose points are (., j0, j1), (j0, ., j1), (j0, j1, .)
+  __device__ static __forceinline__ int line(int d, int j0, int j1)
+  {
+    return d == 0 ? S1 * j0 + S2 * j1 : (d == 1 ? j0 + S2 * j1 : j0 + S1 * j1);
   }
-}
-
-__device__ __forceinline__ int code_u0(int c) { return c & 255; }
-__device__ __forceinline__ int code_st(int c) { return (c >> 8) & 255; }
-__device__ __forceinline__ int code_ax(int c) { return (c >> 16) & 3; }
-__device__ __forceinline__ bool code_plus(int c) { return (c >> 18) & 1; }
-
-// line_interp with the line taken from a flux-point code
-template <int P, typename T, typename S>
-__device__ __forceinline__ T interp_code(const Line<T>& L, int c, const S* s)
-{
-  const int u0 = code_u0(c), st = code_st(c);
-  const bool plus = code_plus(c);
-  T acc = T(0);
-#pragma unroll
-  for (int m = 0; m <= P; m++) acc = acc + (T)s[u0 + m * st] * (plus ? L.Lp[m] : L.Lm[m]);
-  return acc;
-}
-
-// Dynamic shared-memory sizes of the stage kernels.
-template <int DIM, int P, bool ALIAS> struct GradPlan;
-template <int DIM, int P, int EPB, typename TC, int LES = 0, bool ALIAS = false>
-__host__ __device__ constexpr size_t grad_smem_bytes();
-template <int DIM, int P, int EPB, int NT, int VISC, int MODE, typename TC> struct UpdPlan;
-template <int DIM, int P, int EPB, int NT, int VISC, int MODE, typename TC>
-__host__ __device__ constexpr size_t update_smem_bytes();
+  // slot of point r of a run of whole elements
+  __device__ static __forceinline__ int run(int r)
+  {
+    if constexpr (DIM == 3 && S2 != N1 * N1) return (r / PLANE) * S2 + r % PLANE;
+    else return r;
+  }
+};
 
 template <int NT, int ITEMS>
 struct Items {
@@ -276,25 +245,49 @@ __device__ __forceinline__ void lds_line(const T* s, T (&v)[N])
   }
 }
 
-// Shared-memory slot of solution point u in the gradient kernel's per-field
-// point arrays.  Hexahedra of P = 3 in FP64 store point (a, b, c) at
-// 16 c + 4 ((b + c) & 3) + ((a + c) & 3): every z-plane stays one 128-byte
-// row, and the 16 points of any face plane (c, b or a fixed) fall in 16
-// distinct 8-byte bank pairs, so the flux-point phases -- one thread per
-// flux point, 16 threads per face, reading the line through their point --
-// and the line reads of the solution-point phases are free of bank
-// conflicts.  Other shapes, and 4-byte values (32 per bank row), keep the
-// natural order.
-template <int DIM, int P, typename TC>
-__host__ __device__ constexpr bool swz_on()
+template <int N, typename T>
+__device__ __forceinline__ void sts_line(T* s, const T (&v)[N])
 {
-  return DIM == 3 && P == 3 && sizeof(TC) == 8;
+  if constexpr (sizeof(T) == 8 && N % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) *reinterpret_cast<double2*>(s + i) = make_double2(v[i], v[i + 1]);
+  } else if constexpr (sizeof(T) == 4 && N % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(s + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i++) s[i] = v[i];
+  }
 }
-template <int DIM, int P, typename TC>
-__device__ __forceinline__ int swz(int u)
+
+// N values of a line of stride ST (16-byte accesses along x where the rows allow)
+template <int N, int ST, typename T>
+__device__ __forceinline__ void lds_strided(const T* s, T (&v)[N])
 {
-  if constexpr (swz_on<DIM, P, TC>()) return (u & 48) | ((((u >> 2) + (u >> 4)) & 3) << 2) | ((u + (u >> 4)) & 3);
-  else return u;
+  if constexpr (ST == 1) lds_line<N, T>(s, v);
+  else {
+#pragma unroll
+    for (int i = 0; i < N; i++) v[i] = s[i * ST];
+  }
+}
+template <int N, int ST, typename T>
+__device__ __forceinline__ void sts_strided(T* s, const T (&v)[N])
+{
+  if constexpr (ST == 1) sts_line<N, T>(s, v);
+  else {
+#pragma unroll
+    for (int i = 0; i < N; i++) s[i * ST] = v[i];
+  }
+}
+
+// Contiguous run of n values to shared memory, V values per copy and the
+// remainder one by one (dst and src 16-byte aligned where V > 1).
+template <int V, int NT, typename T>
+__device__ __forceinline__ void cp_run(T* dst, const T* src, int n)
+{
+  for (int i = threadIdx.x; i < n / V; i += NT) cp_async<(int)sizeof(T) * V>(dst + i * V, src + i * V);
+  if constexpr (V > 1)
+    for (int i = n / V * V + threadIdx.x; i < n; i += NT) cp_async<(int)sizeof(T)>(dst + i, src + i);
 }
 
 // Boundary points of the gradient kernel, out of line so that the hot loop
@@ -346,61 +339,31 @@ __device__ __noinline__ void vis_boundary(PhysT<TC> ph, int type, BdyPoint<D, TC
   }
 }
 
-// side bytes of the block's flux points, after the operator copy
-template <int EPB, int NF>
-__host__ __device__ constexpr size_t grad_side_bytes()
-{
-  return (EPB * NF + 15) / 16 * 16;
-}
-
-// Shared-memory plan of fr_grad_kernel, per element, in units of TC:
-//   sU  [F][NU]      solution
-//   sX  [F][NF]      neighbour traces, then (in place) delta_disu_fpts
-//   sUf [F][NF]      own solution at the flux points
-//   sM  [R3N]        metrics JGinv (NU x D*D, the reference's per-element
-//                    order) and detJ (NU) for the solution-point phase, then
-//                    the left normals [D][NF] for the flux-point phase
-//   sG  [F*D][NU]    physical gradient (component k + F*d)
-//   sFl [D][F][NU]   transformed total flux
-//   sS  [(F-1)*D][NU] transformed SGS flux (LES only)
-// Every region size is rounded up to 4 words, so each region, and each
-// element's block, starts on a 16-byte boundary whatever the point counts.
-// With ALIAS the transformed flux sFl takes the place of sX and the metrics
-// (both dead once every thread has finished its solution-point reads; the
-// kernel puts a barrier there) and the left normals go to sU (dead after the
-// solution-point phase): 25 % less shared memory per element.  oN is where
-// the left normals [D][NF] live for the flux-point phase.
-template <int DIM, int P, bool ALIAS>
+// Shared-memory plan of fr_grad_kernel, in words of TC; "per point" arrays are
+// [component][element][PtMap::N]:
+//   oF0  state [F], then (each point's own thread overwrites it) the
+//        transformed flux along axis 0, then the running divergence
+//   oF1  transformed flux along axes 1 .. D-1
+//   oM   JGinv (the reference's order, element after element), then detJ
+//   oG   reference gradient, then in place the physical gradient [F*D]
+//   oUf  own solution at the flux points [F][element][NF]
+//   oS   transformed SGS flux [(F-1)*D] (LES only)
+// Region sizes are rounded up to 4 words: every region starts on 16 bytes.
+template <int DIM, int P, int EPB, typename TC>
 struct GradPlan {
   using S = Shape<DIM, P>;
   __host__ __device__ static constexpr int r4(int n) { return (n + 3) / 4 * 4; }
-  static constexpr int NM = (DIM * DIM + 1) * S::NU;        // metrics
-  static constexpr int R3N = ALIAS ? NM : (NM > DIM * S::NF ? NM : DIM * S::NF);
-  static constexpr int oX = r4(S::F * S::NU);
-  static constexpr int oUf = ALIAS ? oX + r4(S::F * S::NF) + r4(R3N) : oX + r4(S::F * S::NF);
-  static constexpr int oM = ALIAS ? oX + r4(S::F * S::NF) : oUf + r4(S::F * S::NF);
-  static constexpr int oG = ALIAS ? oUf + r4(S::F * S::NF) : oM + r4(R3N);
-  static constexpr int oFl = ALIAS ? oX : oG + r4(S::F * DIM * S::NU);
-  static constexpr int oS = ALIAS ? oG + r4(S::F * DIM * S::NU) : oFl + r4(S::F * DIM * S::NU);
-  static constexpr int oN = ALIAS ? 0 : oM;
-  static_assert(!ALIAS || (S::F * DIM * S::NU <= oUf - oX && DIM * S::NF <= oX), "aliased regions too small");
-  __host__ __device__ static constexpr int size(int les) { return oS + (les ? r4((S::F - 1) * DIM * S::NU) : 0); }
+  static constexpr int NW = EPB * PtMap<DIM, P, TC>::N;
+  static constexpr int oF0 = 0, oF1 = oF0 + r4(S::F * NW), oM = oF1 + r4((DIM - 1) * S::F * NW);
+  static constexpr int oDJ = oM + r4(EPB * DIM * DIM * S::NU), oG = oDJ + r4(EPB * S::NU);
+  static constexpr int oUf = oG + r4(S::F * DIM * NW), oS = oUf + r4(S::F * EPB * S::NF);
+  __host__ __device__ static constexpr int size(int les) { return oS + (les ? r4((S::F - 1) * DIM * NW) : 0); }
 };
 
-template <int DIM, int P, int EPB, typename TC, int LES, bool ALIAS>
+template <int DIM, int P, int EPB, typename TC, int LES = 0>
 __host__ __device__ constexpr size_t grad_smem_bytes()
 {
-  return blockops_bytes<TC, Shape<DIM, P>::NF>() + grad_side_bytes<EPB, Shape<DIM, P>::NF>() +
-         sizeof(TC) * EPB * GradPlan<DIM, P, ALIAS>::size(LES);
-}
-
-// Whether an instantiation of fr_grad_kernel uses the aliased shared-memory
-// plan: the FP64 hex P = 3 layout, no LES, not persistent, one solution
-// point per thread (the in-phase barrier needs every thread's reads done).
-template <int DIM, int P, int EPB, int NT, typename TC, int LES, int PERS>
-__host__ __device__ constexpr bool grad_alias()
-{
-  return swz_on<DIM, P, TC>() && LES == 0 && PERS == 0 && Items<NT, EPB * Shape<DIM, P>::NU>::N == 1;
+  return sizeof(TC) * GradPlan<DIM, P, EPB, TC>::size(LES);
 }
 
 // Viscous stage, part 1 (per element):
@@ -421,16 +384,24 @@ __host__ __device__ constexpr bool grad_alias()
 // points (evaluate_sgsFlux, src/eles.cpp:3294-3368) and added there to the
 // physical viscous flux before the projection, as calculate_common_viscFlux
 // adds sgsf_fpts (src/int_inters.cpp:415-427).
-// Inputs reach shared memory through cp.async, so no register holds a
-// prefetched value across the phases; the left normals are fetched while the
-// divergence is computed.  MINB is the CTAs per SM the registers are sized
-// for; VEC = 0 keeps every global read element-sized (inputs only 8-byte
-// aligned), VEC = 1 uses 16-byte copies where the per-element runs allow;
-// PERS = 1 makes the blocks persistent (see the input staging below).
-// Hexahedra of P = 3 in FP64 keep their per-point arrays in the order of swz
-// (bank-conflict-free line reads), run the flux-point phase one line of
-// solution points per task (both end flux points from one read), and, with
-// one point per thread, use the aliased shared-memory plan of GradPlan.
+//
+// Work split.  The line contractions (traces, reference gradient, divergence,
+// normal flux) are one (field, element, line) task per thread and axis: the
+// line's values are read once, its operator rows are compile-time entries of
+// the constant bank, and the element's fields fill F warps or more; the
+// pointwise fluxes are one solution point or flux point per thread, taking the
+// gradient one column at a time, so that 80 registers hold a point (a line's
+// two flux points per thread, and whole gradients, took 128).  Bound: FP64
+// issue, 60 k FP64 instructions per hex P = 3 element (948 cycles of an SM).
+// One output per thread instead, each reading its line and its operator row
+// from shared memory behind run-time index arithmetic, took 5.5 k warp
+// instructions per element of which a third were FP64.
+// The neighbours' traces go to registers (two dependent loads, issued before
+// the wait for the staged state); state, JGinv and detJ reach shared memory
+// through cp.async.  VEC = 0 keeps every global read element-sized (inputs
+// only 8-byte aligned); PERS = 1 makes the blocks persistent: they walk over
+// element blocks blk0, blk0 + bstride, ...; MINB is the CTAs per SM the
+// registers are sized for.
 // Outputs VF (n_fpts, n_eles, F-1), ND (n_fpts, n_eles, F), DV (n_upts, n_eles, F),
 // BV (n_boundary_points, F) the viscous normal flux at boundary points (side
 // bits 2.. hold the boundary type, mate = -1 - position in the boundary
@@ -449,553 +420,364 @@ fr_grad_body(long long blk0, long long bstride, const double* __restrict__ U, co
              TC* __restrict__ BV)
 {
   using S = Shape<DIM, P>;
-  constexpr bool ALIAS = grad_alias<DIM, P, EPB, NT, TC, LES, PERS>();
-  using G = GradPlan<DIM, P, ALIAS>;
-  constexpr int NU = S::NU, NF = S::NF, F = S::F, D = DIM, DD = DIM * DIM;
-  constexpr int IF = Items<NT, EPB * NF>::N, IU = Items<NT, EPB * NU>::N;
-  constexpr int PE = G::size(LES);      // shared TC words per element
+  using G = GradPlan<DIM, P, EPB, TC>;
+  using M = PtMap<DIM, P, TC>;
+  constexpr int N1 = P + 1, NU = S::NU, NF = S::NF, F = S::F, D = DIM, DD = DIM * DIM, NW = G::NW;
+  constexpr int NLN = NU / N1;                      // lines per axis
+  constexpr int LT = F * EPB * NLN;                 // (field, element, line) tasks per axis
+  constexpr int IU = Items<NT, EPB * NU>::N, IF = Items<NT, EPB * NF>::N;
+  static_assert(NT >= LT, "one line task per thread");
   extern __shared__ __align__(16) unsigned char fr_smem[];
-  auto B = reinterpret_cast<BlockOps<TC, NF>*>(fr_smem);
-  unsigned char* sSide = fr_smem + blockops_bytes<TC, NF>();
-  TC* sm = reinterpret_cast<TC*>(fr_smem + blockops_bytes<TC, NF>() + grad_side_bytes<EPB, NF>());
-#define FR_SU(el, k, u) sm[(el) * PE + (k) * NU + (u)]
-#define FR_SX(el, k, f) sm[(el) * PE + G::oX + (k) * NF + (f)]
-#define FR_SUF(el, k, f) sm[(el) * PE + G::oUf + (k) * NF + (f)]
-#define FR_SM(el, i) sm[(el) * PE + G::oM + (i)]
-#define FR_SG(el, c, u) sm[(el) * PE + G::oG + (c) * NU + (u)]
-#define FR_SFL(el, l, k, u) sm[(el) * PE + G::oFl + ((l) * F + (k)) * NU + (u)]
-#define FR_SS(el, c, u) sm[(el) * PE + G::oS + (c) * NU + (u)]
-#define FR_SN(el, i) sm[(el) * PE + G::oN + (i)]
-  fill_blockops<DIM, P, TC, NF>(B, L, threadIdx.x, NT);
+  TC* sm = reinterpret_cast<TC*>(fr_smem);
+  TC* sF0 = sm + G::oF0;
+  TC* sJ = sm + G::oM;
+  TC* sDJ = sm + G::oDJ;
+  TC* sG = sm + G::oG;
+  TC* sUf = sm + G::oUf;
+  TC* sS = sm + G::oS;
+  auto flux = [&](int l, int k, int el) { return sm + (l == 0 ? G::oF0 : G::oF1 + (l - 1) * F * NW) + k * NW + el * M::N; };
+  auto grad = [&](int k, int d, int el) { return sG + (k + F * d) * NW + el * M::N; };
+  const int tid = threadIdx.x;
   const long long NFE = (long long)NF * E;
-  const long long nblk = (E + EPB - 1) / EPB;
-
-  // --- inputs to shared memory: state, metrics, neighbour traces.  16-byte
-  // copies where the per-element runs are whole 16-byte units (global bases
-  // 16-byte aligned), element-sized otherwise.  With PERS = 1 a block walks
-  // over element blocks blk0, + bstride, ...; the next block's state,
-  // metrics and neighbour traces are fetched into their regions as soon as
-  // the current block no longer reads them (after the solution-point phase),
-  // so the copies overlap the divergence and flux-point phases, and the left
-  // normals are read from global memory at the flux points.
-  constexpr bool SWZ = swz_on<DIM, P, TC>();
-  constexpr int VU = (VEC && !SWZ && sizeof(TC) == 8 && NU % 2 == 0) ? 2 : 1;
-  constexpr int VJ = (VEC && (DD * NU * sizeof(TC)) % 16 == 0) ? 16 / sizeof(TC) : 1;
-  constexpr int VD = (VEC && (NU * sizeof(TC)) % 16 == 0) ? 16 / sizeof(TC) : 1;
-  // state (FP64 form: asynchronous; FP32 form: loaded and rounded here)
-  auto stage_state = [&](long long eb, int nv) {
-    for (int w = threadIdx.x; w < EPB * F * NU / VU; w += NT) {
-      int el = w / (F * NU / VU), r = w * VU - el * F * NU, k = r / NU, u = r - k * NU;
-      if (el < nv) {
-        const double* src = U + u + (size_t)NU * (eb + el + E * k);
-        const int su = swz<DIM, P, TC>(u);
-        if constexpr (sizeof(TC) == 8) cp_async<8 * VU>(&FR_SU(el, k, su), src);
-        else FR_SU(el, k, su) = (TC)*src;
-      } else {
-#pragma unroll
-        for (int v = 0; v < VU; v++) {
-          const int su = swz<DIM, P, TC>(u + v);
-          FR_SU(el, k, su) = TC(1);
-        }
-      }
-    }
-  };
-  auto stage_metrics = [&](long long eb, int nv) {
-    for (int w = threadIdx.x; w < nv * DD * NU / VJ; w += NT) {
-      int el = (w * VJ) / (DD * NU), r = w * VJ - el * DD * NU;
-      cp_async<sizeof(TC) * VJ>(&FR_SM(el, r), JG + (size_t)DD * NU * eb + (size_t)w * VJ);
-    }
-    for (int w = threadIdx.x; w < nv * NU / VD; w += NT) {
-      int el = (w * VD) / NU, u = w * VD - el * NU;
-      cp_async<sizeof(TC) * VD>(&FR_SM(el, DD * NU + u), detj + (size_t)NU * eb + (size_t)w * VD);
-    }
-  };
-  // wiring of the thread's flux points: mate index and side byte
-  auto load_wiring = [&](long long eb, int nv, int (&mt)[IF], unsigned char (&sd)[IF]) {
-#pragma unroll
-    for (int it = 0; it < IF; it++) {
-      int w = threadIdx.x + it * NT, el = w / NF, f = w - el * NF;
-      mt[it] = -1;
-      sd[it] = 0;
-      if (w < EPB * NF && el < nv) {
-        size_t own = f + (size_t)NF * (eb + el);
-        mt[it] = mate[own];
-        sd[it] = side[own];
-      }
-    }
-  };
-  // neighbour traces (boundary points, mate < 0, have none)
-  auto stage_traces = [&](const int (&mt)[IF]) {
-#pragma unroll
-    for (int it = 0; it < IF; it++) {
-      int w = threadIdx.x + it * NT, el = w / NF, f = w - el * NF;
-      if (mt[it] >= 0) {
-#pragma unroll
-        for (int k = 0; k < F; k++) cp_async<sizeof(TC)>(&FR_SX(el, k, f), UF + mt[it] + NFE * k);
-      }
-    }
+  // the thread's line task
+  const int k = tid / (EPB * NLN), kr = tid - k * (EPB * NLN), el = kr / NLN, j = kr - el * NLN;
+  const int j0 = DIM == 3 ? j % N1 : j, j1 = DIM == 3 ? j / N1 : 0;
+  auto end_fpt = [&](int d, int e, int q0, int q1) {
+    int al;
+    return face_fpt<DIM, P>(line_face<DIM>(d, e), d == 0 ? 0 : q0, d == 0 ? q0 : (d == 1 ? 0 : q1), d == 2 ? 0 : q1, al);
   };
 
-  long long blk = blk0;
-  int nval = (int)(E - blk * EPB < EPB ? E - blk * EPB : EPB);
-  unsigned char psd[IF];
+  for (long long blk = blk0;; blk += bstride) {
+  const long long e0 = blk * EPB;
+  const int nval = (int)(E - e0 < EPB ? E - e0 : EPB);
+  const bool line = tid < LT && el < nval;
+
+  // --- inputs: state, metrics (cp.async); the neighbours' traces at both ends
+  // of the thread's lines (boundary points, mate < 0, have none)
   {
-    int mt[IF];
-    stage_state(blk * EPB, nval);
-    stage_metrics(blk * EPB, nval);
-    load_wiring(blk * EPB, nval, mt, psd);
-    stage_traces(mt);
+    constexpr int VU = (VEC && sizeof(TC) == 8 && NU % 2 == 0) ? 2 : 1;
+    constexpr int R = EPB * NU / VU, IS = Items<NT, F * R>::N;
+    double tmp[sizeof(TC) == 8 ? 1 : IS];   // FP32: every load in flight before the first is rounded
+#pragma unroll
+    for (int it = 0; it < IS; it++) {
+      const int w = tid + it * NT, kk = w / R, r = (w - kk * R) * VU;
+      const bool ok = w < F * R && r < nval * NU;
+      const double* src = U + (size_t)NU * (e0 + E * kk) + r;
+      if constexpr (sizeof(TC) == 8) {
+        if (ok) cp_async<8 * VU>(sF0 + kk * NW + M::run(r), src);
+      } else {
+        tmp[it] = ok ? *src : 1.0;
+      }
+    }
+    if constexpr (sizeof(TC) != 8)
+#pragma unroll
+      for (int it = 0; it < IS; it++) {
+        const int w = tid + it * NT, kk = w / R, r = w - kk * R;
+        if (w < F * R && r < nval * NU) sF0[kk * NW + M::run(r)] = (TC)tmp[it];
+      }
+    constexpr int VJ = (VEC && (EPB * DD * NU * sizeof(TC)) % 16 == 0) ? 16 / sizeof(TC) : 1;
+    constexpr int VD = (VEC && (EPB * NU * sizeof(TC)) % 16 == 0) ? 16 / sizeof(TC) : 1;
+    cp_run<VJ, NT>(sJ, JG + (size_t)DD * NU * e0, nval * DD * NU);
+    cp_run<VD, NT>(sDJ, detj + (size_t)NU * e0, nval * NU);
     cp_async_commit();
   }
-  for (;;) {
-  const long long e0 = blk * EPB;
+  // two rounds of loads, each without a branch between them (one round trip
+  // per flux point otherwise): the wiring, then the traces; a boundary point
+  // reads its own trace, which is not used
+  TC un[D][2];
+  unsigned char sd[D][2];
+  {
+    int mt[D][2];
+    const unsigned ob = line ? NF * el : 0;   // block-local: one base per array for the whole block
+#pragma unroll
+    for (int d = 0; d < D; d++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const unsigned own = ob + end_fpt(d, e, j0, j1);
+        mt[d][e] = (mate + NF * e0)[own];
+        sd[d][e] = (side + NF * e0)[own];
+        if (mt[d][e] < 0) mt[d][e] = (int)(NF * e0 + own);
+      }
+    const TC* uk = UF + (line ? NFE * k : 0);
+#pragma unroll
+    for (int d = 0; d < D; d++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) un[d][e] = uk[mt[d][e]];
+  }
   cp_async_wait_all();
   __syncthreads();
-#pragma unroll
-  for (int it = 0; it < IF; it++) {
-    const int w = threadIdx.x + it * NT;
-    if (w < EPB * NF) sSide[w] = psd[it];
-  }
 
-  // --- LDG common solution u_c = (uL+uR)/2 - beta (uL-uR); delta = u_c - u_own (in place)
+  // --- lines: own traces, LDG common solution u_c = (uL+uR)/2 - beta (uL-uR),
+  // delta = u_c - u_own, corrected reference gradient along the line (FMAs: it
+  // only feeds the viscous flux)
+  if (line) {
 #pragma unroll
-  for (int it = 0; it < IF; it++) {
-    int w = threadIdx.x + it * NT, el = w / NF, f = w - el * NF;
-    if (w >= EPB * NF || el >= nval) continue;
-    const int cd = B->code[f];
-    int sl[P + 1];
-    TC Lc[P + 1];
+    for (int d = 0; d < D; d++) {
+      const int base = M::line(d, j0, j1);
+      TC v[N1], dl[2];
+      if (d == 0) lds_strided<N1, M::stride(0)>(sF0 + k * NW + el * M::N + base, v);
+      else if (d == 1) lds_strided<N1, M::stride(1)>(sF0 + k * NW + el * M::N + base, v);
+      else lds_strided<N1, M::stride(2)>(sF0 + k * NW + el * M::N + base, v);
 #pragma unroll
-    for (int m = 0; m <= P; m++) {
-      sl[m] = swz<DIM, P, TC>(code_u0(cd) + m * code_st(cd));
-      Lc[m] = code_plus(cd) ? L.Lp[m] : L.Lm[m];
-    }
-    // the reference's opp_0 row of f in column order, (((0 + t0) + t1) + ...)
-    auto trace = [&](int k) {
-      TC acc = TC(0);
+      for (int e = 0; e < 2; e++) {
+        const int f = end_fpt(d, e, j0, j1);
+        // the reference's opp_0 row of f in column order, (((0 + t0) + t1) + ...)
+        TC uo = TC(0);
 #pragma unroll
-      for (int m = 0; m <= P; m++) acc = acc + FR_SU(el, k, sl[m]) * Lc[m];
-      return acc;
-    };
-    if (BV && (psd[it] >> 2)) {
-      BdyPoint<D, TC> q;
+        for (int m = 0; m <= P; m++) uo = uo + v[m] * (e ? L.Lp[m] : L.Lm[m]);
+        sUf[(k * EPB + el) * NF + f] = uo;
+        if (BV && (sd[d][e] >> 2)) {
+          BdyPoint<D, TC> q;
+          TC dx[F], uf[F];
 #pragma unroll
-      for (int k = 0; k < F; k++) q.u[k] = trace(k);
-      const size_t own = f + (size_t)NF * (e0 + el);
+          for (int kk = 0; kk < F; kk++) {
+            TC t = TC(0);
 #pragma unroll
-      for (int d = 0; d < D; d++) q.n[d] = nL[own + NFE * d];
-      ldg_boundary<D, TC>(ph, psd[it] >> 2, q, &FR_SX(el, 0, f), &FR_SUF(el, 0, f), NF);
-      continue;
-    }
-    TC pen = (psd[it] & 2) ? -ph.pen_fact : ph.pen_fact;
+            for (int m = 0; m <= P; m++)
+              t = t + sF0[kk * NW + el * M::N + base + m * M::stride(d)] * (e ? L.Lp[m] : L.Lm[m]);
+            q.u[kk] = t;
+          }
+          const size_t own = f + (size_t)NF * (e0 + el);
 #pragma unroll
-    for (int k = 0; k < F; k++) {
-      TC uo = trace(k);
-      TC un = FR_SX(el, k, f);
-      TC ul = (psd[it] & 1) ? uo : un, ur = (psd[it] & 1) ? un : uo;
-      TC uc = TC(0.5) * (ul + ur) - pen * (ul - ur);
-      FR_SX(el, k, f) = uc - uo;
-      FR_SUF(el, k, f) = uo;
+          for (int dd = 0; dd < D; dd++) q.n[dd] = nL[own + NFE * dd];
+          ldg_boundary<D, TC>(ph, sd[d][e] >> 2, q, dx, uf, 1);
+          dl[e] = dx[k];
+          continue;
+        }
+        // the jump u_l - u_r changes its sign with the side (bit 0: left), as
+        // the penalty does with bit 1
+        const int sb = sd[d][e] & 3;
+        const TC pen = (sb == 1 || sb == 2) ? ph.pen_fact : -ph.pen_fact;
+        dl[e] = (TC(0.5) * (uo + un[d][e]) - pen * (uo - un[d][e])) - uo;
+      }
+      TC g[N1];
+#pragma unroll
+      for (int i = 0; i < N1; i++) {
+        TC acc = v[0] * L.D[i][0];
+#pragma unroll
+        for (int m = 1; m <= P; m++) acc = fr_fma(v[m], L.D[i][m], acc);
+        acc = fr_fma(dl[0], L.gL[i], acc);
+        g[i] = fr_fma(dl[1], L.gR[i], acc);
+      }
+      if (d == 0) sts_strided<N1, M::stride(0)>(grad(k, d, el) + base, g);
+      else if (d == 1) sts_strided<N1, M::stride(1)>(grad(k, d, el) + base, g);
+      else sts_strided<N1, M::stride(2)>(grad(k, d, el) + base, g);
     }
   }
   __syncthreads();
 
-  // --- gradient and total flux at the solution points
+  // --- points: physical gradient and total flux
 #pragma unroll
   for (int it = 0; it < IU; it++) {
-    int w = threadIdx.x + it * NT, el = w / NU, u = w - el * NU;
-    const bool valid = w < EPB * NU && el < nval;
-    if (!ALIAS && !valid) continue;
-    if (!valid) el = u = 0;                  // reads in bounds, results unused
-    int abc[3];
-    upt_abc<DIM, P>(u, abc[0], abc[1], abc[2]);
-    TC gr[F][D];
+    const int w = tid + it * NT, pe = w / NU, u = w - pe * NU;
+    if (w >= EPB * NU || pe >= nval) continue;
+    int a, b, c;
+    upt_abc<DIM, P>(u, a, b, c);
+    const int su = M::slot(a, b, c);
+    TC gr[F][D], q[F];
 #pragma unroll
-    for (int d = 0; d < D; d++) {
-      const int i = abc[d];
-      int fm, fp, am, ap;
-      if (DIM == 2) { fm = d == 0 ? 3 : 0; fp = d == 0 ? 1 : 2; }
-      else { fm = d == 0 ? 4 : (d == 1 ? 1 : 0); fp = d == 0 ? 2 : (d == 1 ? 3 : 5); }
-      int qm = face_fpt<DIM, P>(fm, abc[0], abc[1], abc[2], am);
-      int qp = face_fpt<DIM, P>(fp, abc[0], abc[1], abc[2], ap);
-      const int st = upt_stride<DIM, P>(d), ub = u - i * st;
-      TC Dr[P + 1];
-      int sl[P + 1];
+    for (int kk = 0; kk < F; kk++) {
 #pragma unroll
-      for (int m = 0; m <= P; m++) {
-        Dr[m] = B->D[i][m];
-        sl[m] = swz<DIM, P, TC>(ub + m * st);
-      }
-      const TC gm = B->gL[am], gpl = B->gR[ap];
-#pragma unroll
-      for (int k = 0; k < F; k++) {
-        // the gradient only feeds the viscous flux: contracted with FMAs
-        TC v[P + 1];
-        if (!SWZ && d == 0) lds_line<P + 1, TC>(&FR_SU(el, k, ub), v);
-        else {
-#pragma unroll
-          for (int m = 0; m <= P; m++) v[m] = FR_SU(el, k, sl[m]);
-        }
-        TC acc = v[0] * Dr[0];
-#pragma unroll
-        for (int m = 1; m <= P; m++) acc = fr_fma(v[m], Dr[m], acc);
-        acc = fr_fma(FR_SX(el, k, qm), gm, acc);
-        acc = fr_fma(FR_SX(el, k, qp), gpl, acc);
-        gr[k][d] = acc;
-      }
+      for (int d = 0; d < D; d++) gr[kk][d] = grad(kk, d, pe)[su];
+      q[kk] = sF0[kk * NW + pe * M::N + su];
     }
-    const int su = swz<DIM, P, TC>(u);
-    TC g[DD];
+    const TC* gj = sJ + DD * w;
+    const TC dj = sDJ[w];
+    // physical gradient: d/dx_c = sum_r (JGinv(r,c)/detJ) d/dr
+    // (src/eles.cpp:1822-1878), one column at a time into the viscous flux
+    const TC inv = fr_rcp(dj);
+    VisState<D, TC> vs;
+    vis_begin<D, TC>(ph, q, vs);
+    TC gp[LES ? F : 1][D];
 #pragma unroll
-    for (int q = 0; q < DD; q++) g[q] = FR_SM(el, DD * u + q);
-    const TC dj = FR_SM(el, DD * NU + u);
-    // physical gradient: d/dx_c = sum_r (JGinv(r,c)/detJ) d/dr (src/eles.cpp:1822-1878)
-    TC inv = TC(1.0) / dj;
-    TC gp[F][D];
+    for (int cc = 0; cc < D; cc++) {
+      const TC m0 = gj[0 + D * cc] * inv, m1 = gj[1 + D * cc] * inv, m2 = D == 3 ? gj[2 + D * cc] * inv : TC(0);
+      TC col[F];
 #pragma unroll
-    for (int c = 0; c < D; c++) {
-      TC m0 = g[0 + D * c] * inv, m1 = g[1 + D * c] * inv, m2 = D == 3 ? g[2 + D * c] * inv : TC(0);
-#pragma unroll
-      for (int k = 0; k < F; k++) {
-        TC acc = fr_fma(gr[k][1], m1, gr[k][0] * m0);
-        if (D == 3) acc = fr_fma(gr[k][2], m2, acc);
-        gp[k][c] = acc;
-        if (valid) {
-          FR_SG(el, k + F * c, su) = acc;
-          if (GRAD) GRAD[u + (size_t)NU * (e0 + el + E * (k + (long long)F * c))] = acc;
-        }
+      for (int kk = 0; kk < F; kk++) {
+        TC acc = fr_fma(gr[kk][1], m1, gr[kk][0] * m0);
+        if (D == 3) acc = fr_fma(gr[kk][D - 1], m2, acc);
+        col[kk] = acc;
+        if constexpr (LES != 0) gp[kk][cc] = acc;
+        grad(kk, cc, pe)[su] = acc;
+        if (GRAD) GRAD[u + (size_t)NU * (e0 + pe + E * (kk + (long long)F * cc))] = acc;
       }
+      vis_column<D, TC>(vs, cc, col);
     }
-    TC q[F];
-#pragma unroll
-    for (int k = 0; k < F; k++) q[k] = FR_SU(el, k, su);
-    if constexpr (ALIAS) {
-      // sFl overwrites the neighbour traces and metrics: every thread's reads first
-      __syncthreads();
-      if (!valid) continue;
-    }
-    TC fi[F][D], fv[F][D];
+    TC fi[F][D], fv[F][D], g[DD];
     inv_flux<D, TC>(ph, q, fi);
-    vis_flux_fast<D, TC>(ph, q, gp, fv);
+    vis_flux_end<D, TC>(vs, fv);
+#pragma unroll
+    for (int m = 0; m < DD; m++) g[m] = gj[m];
     if constexpr (LES != 0) {
       TC fs[F][D];
       sgs_flux<D, TC>(ph, q, gp, dj, TC(P + 1), fs);
 #pragma unroll
-      for (int k = 1; k < F; k++)
+      for (int kk = 1; kk < F; kk++)
 #pragma unroll
         for (int l = 0; l < D; l++) {
-          TC a = g[l] * fs[k][0];
+          TC t = g[l] * fs[kk][0];
 #pragma unroll
-          for (int m = 1; m < D; m++) a = a + g[l + D * m] * fs[k][m];
-          FR_SS(el, (k - 1) + (F - 1) * l, su) = a;
-          fv[k][l] = fv[k][l] + fs[k][l];
+          for (int m = 1; m < D; m++) t = t + g[l + D * m] * fs[kk][m];
+          sS[((kk - 1) + (F - 1) * l) * NW + pe * M::N + su] = t;
+          fv[kk][l] = fv[kk][l] + fs[kk][l];
         }
     }
 #pragma unroll
-    for (int k = 0; k < F; k++)
+    for (int kk = 0; kk < F; kk++)
 #pragma unroll
       for (int l = 0; l < D; l++) {
-        // inviscid part in the reference's rounding, viscous part added term by term
-        TC acc = g[l] * fi[k][0];
+        // inviscid part in the reference's rounding, viscous part added term by
+        // term (the density has none)
+        TC acc = g[l] * fi[kk][0];
 #pragma unroll
-        for (int m = 1; m < D; m++) acc = acc + g[l + D * m] * fi[k][m];
+        for (int m = 1; m < D; m++) acc = acc + g[l + D * m] * fi[kk][m];
+        if (kk > 0) {
 #pragma unroll
-        for (int m = 0; m < D; m++) acc = fr_fma(g[l + D * m], fv[k][m], acc);
-        FR_SFL(el, l, k, su) = acc;
+          for (int m = 0; m < D; m++) acc = fr_fma(g[l + D * m], fv[kk][m], acc);
+        }
+        flux(l, kk, pe)[su] = acc;
       }
   }
   __syncthreads();
 
-  // --- the next block's state, metrics and wiring (PERS), or the left
-  // normals into the metric region, fetched while the divergence runs
-  const long long nb = blk + bstride;
-  const bool more = PERS && nb < nblk;
-  const int nvn = more ? (int)(E - nb * EPB < EPB ? E - nb * EPB : EPB) : 0;
-  int mtn[IF];
-  unsigned char psn[IF];
-  if (more) {
-    if constexpr (sizeof(TC) == 8) stage_state(nb * EPB, nvn);
-    stage_metrics(nb * EPB, nvn);
-    load_wiring(nb * EPB, nvn, mtn, psn);
-  }
-  if (!PERS)
-    for (int w = threadIdx.x; w < nval * D * NF; w += NT) {
-      int el = w / (D * NF), r = w - el * D * NF, d = r / NF, f = r - d * NF;
-      cp_async<sizeof(TC)>(&FR_SN(el, r), nL + f + (size_t)NF * (e0 + el) + NFE * d);
+  // the left normal of the thread's flux point, in flight during the divergence
+  const int qe = tid / NF, qf = tid - qe * NF;
+  const bool qlive = tid < EPB * NF && qe < nval;
+  TC nrm[D];
+  if constexpr (IF == 1) {
+    if (qlive) {
+#pragma unroll
+      for (int d = 0; d < D; d++) nrm[d] = (nL + NF * e0 + NFE * d)[(unsigned)tid];
     }
-  cp_async_commit();
+  }
 
-  // --- divergence of the total discontinuous flux
+  // --- lines: divergence of the total discontinuous flux (the reference's
+  // sum_d opp_2[d] row, axes in order: the running sum is kept in place of
+  // the flux along axis 0) and the discontinuous normal flux at both ends
+  // (opp_1 rows in column order).  A warp that holds whole elements of one
+  // field needs no block barrier between the axes.
+  constexpr bool WSYNC = 32 % NLN == 0 && (EPB * NLN) % 32 == 0;
 #pragma unroll
-  for (int it = 0; it < IU; it++) {
-    int w = threadIdx.x + it * NT, el = w / NU, u = w - el * NU;
-    if (w >= EPB * NU || el >= nval) continue;
-    int abc[3];
-    upt_abc<DIM, P>(u, abc[0], abc[1], abc[2]);
-    TC Dm[D][P + 1];
-#pragma unroll
-    for (int d = 0; d < D; d++)
-#pragma unroll
-      for (int m = 0; m <= P; m++) Dm[d][m] = B->D[abc[d]][m];
-    int sl[D][P + 1];
-#pragma unroll
-    for (int d = 0; d < D; d++)
-#pragma unroll
-      for (int m = 0; m <= P; m++) sl[d][m] = swz<DIM, P, TC>(u - abc[d] * upt_stride<DIM, P>(d) + m * upt_stride<DIM, P>(d));
-#pragma unroll
-    for (int k = 0; k < F; k++) {
-      TC acc = TC(0);
-#pragma unroll
-      for (int d = 0; d < D; d++) {
-        const int st = upt_stride<DIM, P>(d), ub = u - abc[d] * st;
-        TC v[P + 1];
-        if (!SWZ && d == 0) lds_line<P + 1, TC>(&FR_SFL(el, d, k, ub), v);
-        else {
-#pragma unroll
-          for (int m = 0; m <= P; m++) v[m] = FR_SFL(el, d, k, sl[d][m]);
-        }
-#pragma unroll
-        for (int m = 0; m <= P; m++) acc = acc + v[m] * Dm[d][m];
-      }
-      DV[u + (size_t)NU * (e0 + el + E * k)] = acc;
-    }
-  }
-  if (more) {
-    stage_traces(mtn);
-    cp_async_commit();
-  }
-  if (!PERS) cp_async_wait_all();
-  __syncthreads();
-
-  if constexpr (SWZ) {
-    // --- flux points, one line of solution points per task: the corrected
-    // gradient (and SGS flux) and the transformed flux along the line are read
-    // once and extrapolated to the flux points at both ends; each end then gets
-    // its own viscous flux projected on the left normal (VF, or BV at a
-    // boundary point) and its discontinuous normal flux ND.
-    constexpr int NLN = NU / (P + 1);               // lines per axis
-    constexpr int IL = Items<NT, EPB * D * NLN>::N;
-#pragma unroll
-    for (int it = 0; it < IL; it++) {
-      const int w = threadIdx.x + it * NT, el = w / (D * NLN), r = w - el * (D * NLN), ax = r / NLN, j = r - ax * NLN;
-      if (w >= EPB * D * NLN || el >= nval) continue;
-      int a = 0, b = 0, c = 0;
-      if (DIM == 2) {
-        if (ax == 0) b = j; else a = j;
-      } else {
-        const int j0 = j % (P + 1), j1 = j / (P + 1);
-        if (ax == 0) { b = j0; c = j1; } else if (ax == 1) { a = j0; c = j1; } else { a = j0; b = j1; }
-      }
-      const int st = upt_stride<DIM, P>(ax), ub = a + (P + 1) * (b + (P + 1) * c);
-      const int fcm = DIM == 2 ? (ax == 0 ? 3 : 0) : (ax == 0 ? 4 : (ax == 1 ? 1 : 0));
-      const int fcp = DIM == 2 ? (ax == 0 ? 1 : 2) : (ax == 0 ? 2 : (ax == 1 ? 3 : 5));
-      int al;
-      const int fe[2] = {face_fpt<DIM, P>(fcm, a, b, c, al), face_fpt<DIM, P>(fcp, a, b, c, al)};
-      int sl[P + 1];
-#pragma unroll
-      for (int m = 0; m <= P; m++) sl[m] = swz<DIM, P, TC>(ub + m * st);
-      // the own corrected gradient at both ends, opp_6 rows in column order with FMAs
-      TC ge[2][F][D];
-#pragma unroll
-      for (int k = 0; k < F; k++)
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-          const TC* s = &FR_SG(el, k + F * d, 0);
-          TC v[P + 1];
-#pragma unroll
-          for (int m = 0; m <= P; m++) v[m] = s[sl[m]];
-          TC am = v[0] * L.Lm[0], ap = v[0] * L.Lp[0];
-#pragma unroll
-          for (int m = 1; m <= P; m++) {
-            am = fr_fma(v[m], L.Lm[m], am);
-            ap = fr_fma(v[m], L.Lp[m], ap);
-          }
-          ge[0][k][d] = am;
-          ge[1][k][d] = ap;
-        }
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int f = fe[e];
-        const size_t own = f + (size_t)NF * (e0 + el);
-        TC uf[F], n[D];
-#pragma unroll
-        for (int k = 0; k < F; k++) uf[k] = FR_SUF(el, k, f);
-#pragma unroll
-        for (int d = 0; d < D; d++) n[d] = PERS ? nL[own + NFE * d] : FR_SN(el, d * NF + f);
-        const int btype = BV ? sSide[el * NF + f] >> 2 : 0;
-        if constexpr (LES == 0) {
-          // the projection is accumulated as the flux is formed (no full flux held)
-          if (btype) {
-            BdyPoint<D, TC> q;
-#pragma unroll
-            for (int k = 0; k < F; k++) {
-              q.u[k] = uf[k];
-#pragma unroll
-              for (int d = 0; d < D; d++) q.g[k][d] = ge[e][k][d];
-            }
-#pragma unroll
-            for (int d = 0; d < D; d++) q.n[d] = n[d];
-            vis_boundary<D, TC, false>(ph, btype, q, &BV[(-1 - (long long)mate[own]) * F]);
-          } else {
-            TC pr[F - 1];
-            vis_flux_proj<D, TC>(ph, uf, ge[e], n, pr);
-#pragma unroll
-            for (int k = 1; k < F; k++) VF[own + NFE * (k - 1)] = pr[k - 1];
-          }
-        } else {
-          TC fv[F][D];
-          vis_flux_fast<D, TC>(ph, uf, ge[e], fv);
-#pragma unroll
-          for (int k = 1; k < F; k++)
-#pragma unroll
-            for (int d = 0; d < D; d++) {
-              const TC* s = &FR_SS(el, (k - 1) + (F - 1) * d, 0);
-              const TC* Lc = e ? L.Lp : L.Lm;
-              TC acc = s[sl[0]] * Lc[0];
-#pragma unroll
-              for (int m = 1; m <= P; m++) acc = fr_fma(s[sl[m]], Lc[m], acc);
-              fv[k][d] = fv[k][d] + acc;
-            }
-          if (btype) {
-            BdyPoint<D, TC> q;
-#pragma unroll
-            for (int k = 0; k < F; k++) {
-              q.u[k] = uf[k];
-#pragma unroll
-              for (int d = 0; d < D; d++) { q.g[k][d] = ge[e][k][d]; q.fv[k][d] = fv[k][d]; }
-            }
-#pragma unroll
-            for (int d = 0; d < D; d++) q.n[d] = n[d];
-            vis_boundary<D, TC>(ph, btype, q, &BV[(-1 - (long long)mate[own]) * F]);
-          } else {
-#pragma unroll
-            for (int k = 1; k < F; k++) VF[own + NFE * (k - 1)] = project<D, TC>(fv, k, n);
-          }
-        }
-      }
-      // the discontinuous normal flux at both ends, opp_1 rows in column order
-      const size_t om = fe[0] + (size_t)NF * (e0 + el), op = fe[1] + (size_t)NF * (e0 + el);
-#pragma unroll
-      for (int k = 0; k < F; k++) {
-        const TC* s = &FR_SFL(el, ax, k, 0);
-        TC vm = TC(0), vp = TC(0);
-#pragma unroll
-        for (int m = 0; m <= P; m++) {
-          const TC x = s[sl[m]];
-          vm = vm + x * L.Lm[m];
-          vp = vp + x * L.Lp[m];
-        }
-        ND[om + NFE * k] = -vm;
-        ND[op + NFE * k] = vp;
-      }
-    }
-  } else {
-    // --- flux points, one thread per flux point: own viscous flux projected on
-    //     the left normal, and the discontinuous normal flux
-#pragma unroll
-    for (int it = 0; it < IF; it++) {
-      int w = threadIdx.x + it * NT, el = w / NF, f = w - el * NF;
-      if (w >= EPB * NF || el >= nval) continue;
-      size_t own = f + (size_t)NF * (e0 + el);
-      TC uf[F], gf[F][D], n[D];
-      const int cd = B->code[f];
-      const int u0 = code_u0(cd), st = code_st(cd), ax = code_ax(cd);
-      const bool plus = code_plus(cd);
-      TC Lc[P + 1];
-      int sl[P + 1];
+  for (int d = 0; d < D; d++) {
+    if (line) {
+      const int base = M::line(d, j0, j1);
+      const size_t oe = (size_t)NF * (e0 + el) + NFE * k;
+      TC v[N1], acc[N1];
+      TC* run = sF0 + k * NW + el * M::N + base;
+      if (d == 0) lds_strided<N1, M::stride(0)>(run, v);
+      else if (d == 1) lds_strided<N1, M::stride(1)>(flux(d, k, el) + base, v);
+      else lds_strided<N1, M::stride(2)>(flux(d, k, el) + base, v);
+      TC vm = TC(0), vp = TC(0);
 #pragma unroll
       for (int m = 0; m <= P; m++) {
-        Lc[m] = plus ? L.Lp[m] : L.Lm[m];
-        sl[m] = swz<DIM, P, TC>(u0 + m * st);
+        vm = vm + v[m] * L.Lm[m];
+        vp = vp + v[m] * L.Lp[m];
+      }
+      ND[oe + end_fpt(d, 0, j0, j1)] = -vm;
+      ND[oe + end_fpt(d, 1, j0, j1)] = vp;
+      if (d == 1) lds_strided<N1, M::stride(1)>(run, acc);
+      if (d == 2) lds_strided<N1, M::stride(2)>(run, acc);
+#pragma unroll
+      for (int i = 0; i < N1; i++) {
+        TC t = d == 0 ? TC(0) : acc[i];
+#pragma unroll
+        for (int m = 0; m <= P; m++) t = t + v[m] * L.D[i][m];
+        acc[i] = t;
+      }
+      if (d == D - 1) {
+        TC* out = DV + (size_t)NU * (e0 + el + E * k) + j0 + (DIM == 3 ? N1 * j1 : 0);
+#pragma unroll
+        for (int i = 0; i < N1; i++) out[i * (DIM == 3 ? N1 * N1 : N1)] = acc[i];
+      } else if (d == 0) sts_strided<N1, M::stride(0)>(run, acc);
+      else sts_strided<N1, M::stride(1)>(run, acc);
+    }
+    if (d < D - 1) {
+      if constexpr (WSYNC) __syncwarp();
+      else __syncthreads();
+    }
+  }
+
+  // --- flux points: the own corrected gradient (and SGS flux) extrapolated
+  // along the line through the point (opp_6 rows in column order with FMAs), one
+  // column at a time into the own viscous flux, projected on the left normal
+  // (VF, or BV at a boundary point).
+#pragma unroll
+  for (int it = 0; it < IF; it++) {
+    const int w = tid + it * NT, pe = it ? w / NF : qe, f = it ? w - pe * NF : qf;
+    if (w >= EPB * NF || pe >= nval) continue;
+    const long long own = f + NF * (e0 + pe);
+    int u0, ust, ax, a, b, c;
+    bool plus;
+    fpt_line<DIM, P>(f, u0, ust, ax, plus);
+    upt_abc<DIM, P>(u0, a, b, c);
+    const int base = M::slot(a, b, c) + pe * M::N, st = ax == 0 ? 1 : (ax == 1 ? M::S1 : M::S2);
+    TC uf[F], n[D], Lc[N1];
+#pragma unroll
+    for (int m = 0; m <= P; m++) Lc[m] = plus ? L.Lp[m] : L.Lm[m];
+#pragma unroll
+    for (int kk = 0; kk < F; kk++) uf[kk] = sUf[(kk * EPB + pe) * NF + f];
+#pragma unroll
+    for (int d = 0; d < D; d++) n[d] = IF == 1 ? nrm[d] : nL[own + NFE * d];
+    auto extrap = [&](const TC* s) {
+      TC acc = s[0] * Lc[0];
+#pragma unroll
+      for (int m = 1; m <= P; m++) acc = fr_fma(s[m * st], Lc[m], acc);
+      return acc;
+    };
+    const int btype = BV ? side[own] >> 2 : 0;
+    if (btype) {
+      BdyPoint<D, TC> q;
+#pragma unroll
+      for (int kk = 0; kk < F; kk++) {
+        q.u[kk] = uf[kk];
+#pragma unroll
+        for (int d = 0; d < D; d++) q.g[kk][d] = extrap(sG + (kk + F * d) * NW + base);
       }
 #pragma unroll
-      for (int k = 0; k < F; k++) {
-        uf[k] = FR_SUF(el, k, f);
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-          const TC* s = &FR_SG(el, k + F * d, 0);
-          TC acc = s[sl[0]] * Lc[0];
-#pragma unroll
-          for (int m = 1; m <= P; m++) acc = fr_fma(s[sl[m]], Lc[m], acc);
-          gf[k][d] = acc;
-        }
-      }
-#pragma unroll
-      for (int d = 0; d < D; d++) n[d] = PERS ? nL[own + NFE * d] : FR_SN(el, d * NF + f);
-      const int btype = BV ? psd[it] >> 2 : 0;
+      for (int d = 0; d < D; d++) q.n[d] = n[d];
+      TC* out = &BV[(-1 - (long long)mate[own]) * F];
       if constexpr (LES == 0) {
-        // the projection is accumulated as the flux is formed (no full flux held)
-        if (btype) {
-          BdyPoint<D, TC> q;
-#pragma unroll
-          for (int k = 0; k < F; k++) {
-            q.u[k] = uf[k];
-#pragma unroll
-            for (int d = 0; d < D; d++) q.g[k][d] = gf[k][d];
-          }
-#pragma unroll
-          for (int d = 0; d < D; d++) q.n[d] = n[d];
-          vis_boundary<D, TC, false>(ph, btype, q, &BV[(-1 - (long long)mate[own]) * F]);
-        } else {
-          TC pr[F - 1];
-          vis_flux_proj<D, TC>(ph, uf, gf, n, pr);
-#pragma unroll
-          for (int k = 1; k < F; k++) VF[own + NFE * (k - 1)] = pr[k - 1];
-        }
+        vis_boundary<D, TC, false>(ph, btype, q, out);
       } else {
-        TC fv[F][D];
-        vis_flux_fast<D, TC>(ph, uf, gf, fv);
+        vis_flux_fast<D, TC>(ph, q.u, q.g, q.fv);
 #pragma unroll
-        for (int k = 1; k < F; k++)
+        for (int kk = 1; kk < F; kk++)
 #pragma unroll
-          for (int d = 0; d < D; d++) {
-            const TC* s = &FR_SS(el, (k - 1) + (F - 1) * d, 0);
-            TC acc = s[sl[0]] * Lc[0];
-#pragma unroll
-            for (int m = 1; m <= P; m++) acc = fr_fma(s[sl[m]], Lc[m], acc);
-            fv[k][d] = fv[k][d] + acc;
-          }
-        if (btype) {
-          BdyPoint<D, TC> q;
-#pragma unroll
-          for (int k = 0; k < F; k++) {
-            q.u[k] = uf[k];
-#pragma unroll
-            for (int d = 0; d < D; d++) { q.g[k][d] = gf[k][d]; q.fv[k][d] = fv[k][d]; }
-          }
-#pragma unroll
-          for (int d = 0; d < D; d++) q.n[d] = n[d];
-          vis_boundary<D, TC>(ph, btype, q, &BV[(-1 - (long long)mate[own]) * F]);
-        } else {
-#pragma unroll
-          for (int k = 1; k < F; k++) VF[own + NFE * (k - 1)] = project<D, TC>(fv, k, n);
-        }
+          for (int d = 0; d < D; d++) q.fv[kk][d] = q.fv[kk][d] + extrap(sS + ((kk - 1) + (F - 1) * d) * NW + base);
+        vis_boundary<D, TC>(ph, btype, q, out);
       }
+      continue;
+    }
+    VisState<D, TC> vs;
+    vis_begin<D, TC>(ph, uf, vs);
 #pragma unroll
-      for (int k = 0; k < F; k++) {
-        const TC* s = &FR_SFL(el, ax, k, 0);
-        TC v = TC(0);
+    for (int d = 0; d < D; d++) {
+      TC col[F];
 #pragma unroll
-        for (int m = 0; m <= P; m++) v = v + s[sl[m]] * Lc[m];
-        ND[own + NFE * k] = plus ? v : -v;
+      for (int kk = 0; kk < F; kk++) col[kk] = extrap(sG + (kk + F * d) * NW + base);
+      vis_column<D, TC>(vs, d, col);
+    }
+    if constexpr (LES == 0) {
+      // the projection is accumulated as the flux is formed (no full flux held)
+      TC pr[F - 1];
+      vis_proj_end<D, TC>(vs, n, pr);
+#pragma unroll
+      for (int kk = 1; kk < F; kk++) (VF + NF * e0 + NFE * (kk - 1))[(unsigned)w] = pr[kk - 1];
+    } else {
+      TC fv[F][D];
+      vis_flux_end<D, TC>(vs, fv);
+#pragma unroll
+      for (int kk = 1; kk < F; kk++) {
+#pragma unroll
+        for (int d = 0; d < D; d++) fv[kk][d] = fv[kk][d] + extrap(sS + ((kk - 1) + (F - 1) * d) * NW + base);
+        VF[own + NFE * (kk - 1)] = project<D, TC>(fv, kk, n);
       }
     }
   }
-  if (!more) break;
-  blk = nb;
-  nval = nvn;
-#pragma unroll
-  for (int it = 0; it < IF; it++) psd[it] = psn[it];
-  if constexpr (sizeof(TC) != 8) stage_state(blk * EPB, nval);   // the state region is free after the solution-point phase
+  if (!PERS || (blk + bstride) * EPB >= E) break;
+  __syncthreads();   // this block's arrays have been read
   }
-#undef FR_SU
-#undef FR_SX
-#undef FR_SUF
-#undef FR_SM
-#undef FR_SG
-#undef FR_SFL
-#undef FR_SS
-#undef FR_SN
 }
 
 template <int DIM, int P, int EPB, int NT, typename TC, int LES = 0, int MINB = 1, int VEC = 1, int PERS = 0>
@@ -1156,273 +938,6 @@ fr_face_kernel(const int2* __restrict__ face, const unsigned char* __restrict__ 
                const TC* __restrict__ BV = nullptr)
 {
   fr_face_body<DIM, VISC, TC, RIEMANN>(blockIdx.x, face, fsign, nint, UF, VF, nL, tdA, CF, NFE, ph, nbdy, bf, bt, BV);
-}
-
-// ---------------------------------------------------------------------------
-// Stage, last part (per element): norm_tconf - norm_tdisf, the VCJH
-// correction (calculate_corrected_divergence, src/eles.cpp:1594-1661), and
-// either the residual (MODE 0) or the RK45 stage update
-// (eles::AdvanceSolution, src/eles.cpp:1155-1178) followed by the next
-// stage's traces (MODE 1).  The inviscid path (VISC 0) evaluates the flux,
-// its divergence and its normal component here itself, in the reference's
-// order; the viscous path takes DV and ND from fr_grad_kernel.
-// Shared-memory plan of fr_update_kernel (byte offsets, every region
-// rounded up to 16 bytes): state and RK register (FP64), detJ (FP64), common
-// normal flux CF (overwritten in place by norm_tconf - norm_tdisf), ND and DV
-// (viscous path), transformed flux and JGinv (inviscid path), norm partials.
-template <int DIM, int P, int EPB, int NT, int VISC, int MODE, typename TC>
-struct UpdPlan {
-  using S = Shape<DIM, P>;
-  __host__ __device__ static constexpr size_t r16(size_t b) { return (b + 15) / 16 * 16; }
-  static constexpr size_t bU = r16(sizeof(double) * EPB * S::F * S::NU);
-  static constexpr size_t bREG = MODE == 1 ? bU : 0;
-  static constexpr size_t bDJ = MODE == 1 ? r16(sizeof(double) * EPB * S::NU) : 0;
-  static constexpr size_t bCF = r16(sizeof(TC) * EPB * S::F * S::NF);
-  static constexpr size_t bND = VISC ? bCF : 0;
-  static constexpr size_t bDV = VISC ? r16(sizeof(TC) * EPB * S::F * S::NU) : 0;
-  static constexpr size_t bFL = VISC ? 0 : r16(sizeof(TC) * EPB * DIM * S::F * S::NU);
-  static constexpr size_t bJ = VISC ? 0 : r16(sizeof(TC) * EPB * DIM * DIM * S::NU);
-  static constexpr size_t bRED = r16(sizeof(double) * (NT / 32) * S::F);
-  static constexpr size_t oU = 0, oREG = oU + bU, oDJ = oREG + bREG, oCF = oDJ + bDJ, oND = oCF + bCF,
-                          oDV = oND + bND, oFL = oDV + bDV, oJ = oFL + bFL, oRED = oJ + bJ, total = oRED + bRED;
-};
-
-template <int DIM, int P, int EPB, int NT, int VISC, int MODE, typename TC>
-__host__ __device__ constexpr size_t update_smem_bytes()
-{
-  return blockops_bytes<TC, Shape<DIM, P>::NF>() + UpdPlan<DIM, P, EPB, NT, VISC, MODE, TC>::total;
-}
-
-// Stage, last part (per element): norm_tconf - norm_tdisf, the VCJH
-// correction (calculate_corrected_divergence, src/eles.cpp:1594-1661), and
-// either the residual (MODE 0) or the RK45 stage update
-// (eles::AdvanceSolution, src/eles.cpp:1155-1178) followed by the next
-// stage's traces (MODE 1).  The inviscid path (VISC 0) evaluates the flux,
-// its divergence and its normal component here itself, in the reference's
-// order; the viscous path takes DV and ND from fr_grad_kernel.  Every
-// per-element input reaches shared memory through cp.async (16-byte copies
-// where the element runs allow, VEC = 1; element-sized with VEC = 0 for
-// inputs only 8-byte aligned), so all of a block's loads are in flight
-// together.
-// The body serves element block blk (fr_update_kernel: blockIdx.x; merged
-// batch launches: their share of the grid).
-template <int DIM, int P, int EPB, int NT, int VISC, int MODE, typename TC, int VEC = 1>
-__device__ __forceinline__ void
-fr_update_body(long long blk, double* __restrict__ U, double* __restrict__ REG, TC* __restrict__ UFn,
-               const TC* __restrict__ CF, const TC* __restrict__ ND, const TC* __restrict__ DV,
-               const TC* __restrict__ JG, const double* __restrict__ detj, double* __restrict__ DIV,
-               double* __restrict__ partial, long long E, const Line<TC>& L, const PhysT<TC>& ph, double rk_a,
-               double rk_b, double dt, int first_stage)
-{
-  using S = Shape<DIM, P>;
-  using Q = UpdPlan<DIM, P, EPB, NT, VISC, MODE, TC>;
-  constexpr int NU = S::NU, NF = S::NF, F = S::F, D = DIM, DD = DIM * DIM;
-  extern __shared__ __align__(16) unsigned char fr_smem[];
-  auto B = reinterpret_cast<BlockOps<TC, NF>*>(fr_smem);
-  unsigned char* sm0 = fr_smem + blockops_bytes<TC, NF>();
-  auto sU = reinterpret_cast<double (*)[F][NU]>(sm0 + Q::oU);
-  auto sREG = reinterpret_cast<double (*)[F][NU]>(sm0 + Q::oREG);
-  auto sDJ = reinterpret_cast<double (*)[NU]>(sm0 + Q::oDJ);
-  auto sC = reinterpret_cast<TC (*)[F][NF]>(sm0 + Q::oCF);
-  auto sND = reinterpret_cast<TC (*)[F][NF]>(sm0 + Q::oND);
-  auto sDV = reinterpret_cast<TC (*)[F][NU]>(sm0 + Q::oDV);
-  auto sFl = reinterpret_cast<TC (*)[D][F][NU]>(sm0 + Q::oFL);
-  auto sJ = reinterpret_cast<TC (*)[DD * NU]>(sm0 + Q::oJ);
-  auto sRed = reinterpret_cast<double (*)[F]>(sm0 + Q::oRED);
-  fill_blockops<DIM, P, TC, NF>(B, L, threadIdx.x, NT);
-  const long long e0 = blk * EPB;
-  const int nval = (int)(E - e0 < EPB ? E - e0 : EPB);
-
-  // --- inputs to shared memory
-  constexpr int V8 = (VEC && NU % 2 == 0) ? 2 : 1;                                   // doubles per copy
-  constexpr int VF = (VEC && (NF * sizeof(TC)) % 16 == 0) ? 16 / sizeof(TC) : 1;     // flux-point runs
-  constexpr int VN = (VEC && (NU * sizeof(TC)) % 16 == 0) ? 16 / sizeof(TC) : 1;     // point runs
-  constexpr int VJ = (VEC && (DD * NU * sizeof(TC)) % 16 == 0) ? 16 / sizeof(TC) : 1;
-  // the state is kept in the bank-conflict-free point order of swz (read
-  // along lines for the next stage's traces), so its copies are element-sized
-  // where that order is not the natural one
-  constexpr bool SWU = swz_on<DIM, P, double>();
-  constexpr int V8U = SWU ? 1 : V8;
-  const bool want_reg = MODE == 1 && !first_stage;
-  for (int w = threadIdx.x; w < nval * F * NU / V8U; w += NT) {
-    int el = w / (F * NU / V8U), r = w * V8U - el * F * NU, k = r / NU, u = r - k * NU;
-    cp_async<8 * V8U>(&sU[el][k][swz<DIM, P, double>(u)], U + u + (size_t)NU * (e0 + el + E * k));
-  }
-  if (want_reg)
-    for (int w = threadIdx.x; w < nval * F * NU / V8; w += NT) {
-      int el = w / (F * NU / V8), r = w * V8 - el * F * NU, k = r / NU, u = r - k * NU;
-      cp_async<8 * V8>(&sREG[el][k][u], REG + u + (size_t)NU * (e0 + el + E * k));
-    }
-  if (MODE == 1)
-    for (int w = threadIdx.x; w < nval * NU / V8; w += NT) {
-      int el = (w * V8) / NU, u = w * V8 - el * NU;
-      cp_async<8 * V8>(&sDJ[el][u], detj + (size_t)NU * e0 + (size_t)w * V8);
-    }
-  for (int w = threadIdx.x; w < nval * F * NF / VF; w += NT) {
-    int el = w / (F * NF / VF), r = w * VF - el * F * NF, k = r / NF, f = r - k * NF;
-    size_t g = f + (size_t)NF * (e0 + el + E * k);
-    cp_async<sizeof(TC) * VF>(&sC[el][k][f], CF + g);
-    if (VISC) cp_async<sizeof(TC) * VF>(&sND[el][k][f], ND + g);
-  }
-  if (VISC)
-    for (int w = threadIdx.x; w < nval * F * NU / VN; w += NT) {
-      int el = w / (F * NU / VN), r = w * VN - el * F * NU, k = r / NU, u = r - k * NU;
-      cp_async<sizeof(TC) * VN>(&sDV[el][k][u], DV + u + (size_t)NU * (e0 + el + E * k));
-    }
-  else
-    for (int w = threadIdx.x; w < nval * DD * NU / VJ; w += NT) {
-      int el = (w * VJ) / (DD * NU), r = w * VJ - el * DD * NU;
-      cp_async<sizeof(TC) * VJ>(&sJ[el][r], JG + (size_t)DD * NU * e0 + (size_t)w * VJ);
-    }
-  cp_async_commit();
-  cp_async_wait_all();
-  __syncthreads();
-
-  if (VISC) {
-    for (int w = threadIdx.x; w < nval * F * NF; w += NT) {
-      int el = w / (F * NF), r = w - el * F * NF, k = r / NF, f = r - k * NF;
-      sC[el][k][f] = sC[el][k][f] - sND[el][k][f];      // daxpy(-1, norm_tdisf, norm_tconf)
-    }
-  } else {
-    // transformed inviscid flux at the solution points (evaluate_invFlux, src/eles.cpp:1331-1418)
-    for (int w = threadIdx.x; w < nval * NU; w += NT) {
-      int el = w / NU, u = w - el * NU;
-      TC g[DD];
-#pragma unroll
-      for (int q = 0; q < DD; q++) g[q] = sJ[el][DD * u + q];
-      TC q[F], fi[F][D];
-#pragma unroll
-      for (int k = 0; k < F; k++) q[k] = (TC)sU[el][k][swz<DIM, P, double>(u)];
-      inv_flux<D, TC>(ph, q, fi);
-#pragma unroll
-      for (int l = 0; l < D; l++)
-#pragma unroll
-        for (int k = 0; k < F; k++) {
-          TC acc = g[l] * fi[k][0];
-#pragma unroll
-          for (int m = 1; m < D; m++) acc = acc + g[l + D * m] * fi[k][m];
-          sFl[el][l][k][u] = acc;
-        }
-    }
-    __syncthreads();
-    // norm_tconf - norm_tdisf with the normal component extrapolated here (extrapolate_totalFlux)
-    for (int w = threadIdx.x; w < nval * NF; w += NT) {
-      int el = w / NF, f = w - el * NF;
-      const int cd = B->code[f];
-      const bool plus = code_plus(cd);
-#pragma unroll
-      for (int k = 0; k < F; k++) {
-        TC v = interp_code<P, TC, TC>(L, cd, &sFl[el][code_ax(cd)][k][0]);
-        sC[el][k][f] = sC[el][k][f] - (plus ? v : -v);
-      }
-    }
-  }
-  __syncthreads();
-
-  double red[F];
-#pragma unroll
-  for (int k = 0; k < F; k++) red[k] = 0.0;
-  constexpr int IU = Items<NT, EPB * NU>::N;
-#pragma unroll
-  for (int it = 0; it < IU; it++) {
-    int w = threadIdx.x + it * NT, el = w / NU, u = w - el * NU;
-    if (w >= EPB * NU || el >= nval) continue;
-    const long long e = e0 + el;
-    int abc[3];
-    upt_abc<DIM, P>(u, abc[0], abc[1], abc[2]);
-    // opp_3 row of u: one column per face, in flux-point order (the same for every field)
-    int qf[S::NFACE];
-    TC cf[S::NFACE];
-#pragma unroll
-    for (int fc = 0; fc < S::NFACE; fc++) {
-      int al;
-      qf[fc] = face_fpt<DIM, P>(fc, abc[0], abc[1], abc[2], al);
-      cf[fc] = face_plus<DIM>(fc) ? B->gR[al] : -B->gL[al];
-    }
-    const double dj = MODE == 1 ? sDJ[el][u] : 1.0;
-#pragma unroll
-    for (int k = 0; k < F; k++) {
-      size_t gi = u + (size_t)NU * (e + E * k);
-      TC acc;
-      if (VISC) {
-        acc = sDV[el][k][u];
-      } else {
-        acc = TC(0);
-#pragma unroll
-        for (int d = 0; d < D; d++) {
-          const int st = upt_stride<DIM, P>(d), ub = u - abc[d] * st;
-#pragma unroll
-          for (int m = 0; m <= P; m++) acc = acc + sFl[el][d][k][ub + m * st] * B->D[abc[d]][m];
-        }
-      }
-#pragma unroll
-      for (int fc = 0; fc < S::NFACE; fc++) acc = acc + sC[el][k][qf[fc]] * cf[fc];
-      double R = (double)acc;
-      if (MODE == 0) {
-        DIV[gi] = R;
-      } else {
-        double rhs = -R / dj;
-        double res = first_stage ? dt * rhs : rk_a * sREG[el][k][u] + dt * rhs;
-        REG[gi] = res;
-        const int su = swz<DIM, P, double>(u);
-        double un = sU[el][k][su] + rk_b * res;
-        U[gi] = un;
-        sU[el][k][su] = un;
-        red[k] += fabs(rhs);
-      }
-    }
-  }
-  if (MODE == 1) {
-    if (partial) {
-      // deterministic per-block partial sums of |div/detjac| (CalcNormResidual)
-      const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-      for (int k = 0; k < F; k++) {
-        double v = red[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) sRed[wid][k] = v;
-      }
-    }
-    __syncthreads();
-    if (partial && threadIdx.x < F) {
-      double v = 0.0;
-      for (int i = 0; i < NT / 32; i++) v += sRed[i][threadIdx.x];
-      partial[(size_t)blk * F + threadIdx.x] = v;
-    }
-    // traces of the updated state for the next stage
-    for (int w = threadIdx.x; w < nval * NF; w += NT) {
-      int el = w / NF, f = w - el * NF;
-      long long e = e0 + el;
-      const int cd = B->code[f];
-      int sl[P + 1];
-      TC Lc[P + 1];
-#pragma unroll
-      for (int m = 0; m <= P; m++) {
-        sl[m] = swz<DIM, P, double>(code_u0(cd) + m * code_st(cd));
-        Lc[m] = code_plus(cd) ? L.Lp[m] : L.Lm[m];
-      }
-      // the opp_0 row of f in column order, (((0 + t0) + t1) + ...)
-#pragma unroll
-      for (int k = 0; k < F; k++) {
-        TC acc = TC(0);
-#pragma unroll
-        for (int m = 0; m <= P; m++) acc = acc + (TC)sU[el][k][sl[m]] * Lc[m];
-        UFn[f + (size_t)NF * (e + E * k)] = acc;
-      }
-    }
-  }
-}
-
-template <int DIM, int P, int EPB, int NT, int VISC, int MODE, typename TC, int VEC = 1>
-__global__ void __launch_bounds__(NT)
-fr_update_kernel(double* __restrict__ U, double* __restrict__ REG, TC* __restrict__ UFn, const TC* __restrict__ CF,
-                 const TC* __restrict__ ND, const TC* __restrict__ DV, const TC* __restrict__ JG,
-                 const double* __restrict__ detj, double* __restrict__ DIV, double* __restrict__ partial, long long E,
-                 Line<TC> L, PhysT<TC> ph, double rk_a, double rk_b, double dt, int first_stage)
-{
-  fr_update_body<DIM, P, EPB, NT, VISC, MODE, TC, VEC>(blockIdx.x, U, REG, UFn, CF, ND, DV, JG, detj, DIV, partial, E,
-                                                       L, ph, rk_a, rk_b, dt, first_stage);
 }
 
 // Block partial sums -> norms: one CTA of 256 threads per field; thread t

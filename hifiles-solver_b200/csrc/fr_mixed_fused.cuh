@@ -8,7 +8,7 @@
 
 #include <cuda_runtime.h>
 
-#include "fr_face_update.cuh"
+#include "fr_update.cuh"
 #include "fr_physics.cuh"
 
 namespace frb_mixed {

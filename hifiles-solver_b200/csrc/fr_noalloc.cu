@@ -16,9 +16,10 @@
 #include <cstdint>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "fr_b200.h"
-#include "fr_fused.cuh"
+#include "fr_update.cuh"
 #include "fr_host.hpp"
 
 namespace frb {
@@ -64,17 +65,18 @@ fr_status scratch_for_device(int dev, double** out)
   return FR_OK;
 }
 
-// Default tiles (elements per CTA, threads per CTA) of the element kernels.
+// Tiles (elements per CTA, threads of the gradient and of the update kernel):
+// one line task, solution point and flux point per thread.
 template <int DIM, int P> struct NaTile;
-template <> struct NaTile<2, 1> { static constexpr int EPB = 32, NT = 128; };
-template <> struct NaTile<2, 2> { static constexpr int EPB = 16, NT = 128; };
+template <> struct NaTile<2, 1> { static constexpr int EPB = 16, NT = 128; };
+template <> struct NaTile<2, 2> { static constexpr int EPB = 10, NT = 128; };
 template <> struct NaTile<2, 3> { static constexpr int EPB = 8, NT = 128; };
-template <> struct NaTile<2, 4> { static constexpr int EPB = 8, NT = 256; };
-template <> struct NaTile<2, 5> { static constexpr int EPB = 4, NT = 160; };
-template <> struct NaTile<3, 1> { static constexpr int EPB = 12, NT = 128; };
-template <> struct NaTile<3, 2> { static constexpr int EPB = 4, NT = 128; };
-template <> struct NaTile<3, 3> { static constexpr int EPB = 2, NT = 128; };
-template <> struct NaTile<3, 4> { static constexpr int EPB = 1, NT = 128; };
+template <> struct NaTile<2, 4> { static constexpr int EPB = 5, NT = 128; };
+template <> struct NaTile<2, 5> { static constexpr int EPB = 5, NT = 192; };
+template <> struct NaTile<3, 1> { static constexpr int EPB = 6, NT = 160; };
+template <> struct NaTile<3, 2> { static constexpr int EPB = 4, NT = 224; };
+template <> struct NaTile<3, 3> { static constexpr int EPB = 2, NT = 192; };
+template <> struct NaTile<3, 4> { static constexpr int EPB = 1, NT = 160; };
 
 bool make_line_noalloc(int P, int upts_type, int scheme, double eta_in, Line<double>& L)
 {
@@ -144,23 +146,17 @@ fr_status run(const fr_residual_args* a, double* scratch, cudaStream_t s)
       fr_face_kernel<DIM, 0, double><<<g, 128, 0, s>>>(face, a->face_sign, a->n_int, UF, nullptr, a->norm_left,
                                                        a->tdA_fpts, CF, NFE, ph);
   }
-  if (visc) {
-    constexpr size_t sm = update_smem_bytes<DIM, P, EPB, NT, 1, 0, double>();
-    if (sm > 48 * 1024)
-      cudaFuncSetAttribute(fr_update_kernel<DIM, P, EPB, NT, 1, 0, double, 0>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    fr_update_kernel<DIM, P, EPB, NT, 1, 0, double, 0><<<nblk, NT, sm, s>>>(
-        const_cast<double*>(a->disu_upts), nullptr, nullptr, CF, ND, DV, a->JGinv_upts, a->detjac_upts, a->div_tconf_upts, nullptr, E, L, ph,
-        0.0, 0.0, 0.0, 0);
-  } else {
-    constexpr size_t sm = update_smem_bytes<DIM, P, EPB, NT, 0, 0, double>();
-    if (sm > 48 * 1024)
-      cudaFuncSetAttribute(fr_update_kernel<DIM, P, EPB, NT, 0, 0, double, 0>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    fr_update_kernel<DIM, P, EPB, NT, 0, 0, double, 0><<<nblk, NT, sm, s>>>(
-        const_cast<double*>(a->disu_upts), nullptr, nullptr, CF, nullptr, nullptr, a->JGinv_upts, a->detjac_upts,
-        a->div_tconf_upts, nullptr, E, L, ph, 0.0, 0.0, 0.0, 0);
-  }
+  auto update = [&](auto V) {
+    constexpr int VISC = decltype(V)::value;
+    constexpr size_t sm = update_smem_bytes<DIM, P, EPB, NT, VISC, 0, double>();
+    auto k = fr_update_kernel<DIM, P, EPB, NT, VISC, 0, double, 0, 0, 1, 0>;
+    if (sm > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k<<<nblk, NT, sm, s>>>(const_cast<double*>(a->disu_upts), nullptr, nullptr, nullptr, CF, a->mate, a->side, nullptr,
+                           ND, DV, a->JGinv_upts, nullptr, nullptr, nullptr, nullptr, a->div_tconf_upts, nullptr, E, L,
+                           ph, 0.0, 0.0, 0.0, 0);
+  };
+  if (visc) update(std::integral_constant<int, 1>());
+  else update(std::integral_constant<int, 0>());
   e = cudaGetLastError();
   if (e != cudaSuccess) return na_fail(FR_ERR_CUDA, cudaGetErrorString(e));
   return FR_OK;

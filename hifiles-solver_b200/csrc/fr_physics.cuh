@@ -177,64 +177,84 @@ __device__ __forceinline__ void vis_flux(const PhysT<T>& ph, const T* u, T (*g)[
 // ~1/Re of the inviscid flux they are added to: its ulp-level differences from
 // the reference's division form stay far below the rounding of the total flux.
 
-// Shared part of the viscous flux: velocity v, stress tau and the heat-flux
-// term q[l] = (mu gamma / Pr) de/dx_l of calc_visf_3d (src/flux.cpp:263-431).
+// Shared part of the viscous flux, calc_visf_3d (src/flux.cpp:263-431), taken
+// one column of the gradient at a time so that a caller never holds more than
+// one: vis_begin from the state, vis_column for every direction l with g[k] =
+// d u_k / d x_l, then vis_end for the stress tau and the heat-flux term
+// q[l] = (mu gamma / Pr) de/dx_l.
 template <int D, typename T>
-__device__ __forceinline__ void vis_core(const PhysT<T>& ph, const T* u, T (*g)[D], T (&v)[D], T (&tau)[D][D],
-                                         T (&q)[D])
+struct VisState {
+  T v[D], rho, ri, ke, inte, mu, kg;
+  T dv[D][D], de[D];   // dv[m][l] = d v_m / d x_l
+};
+template <int D, typename T>
+__device__ __forceinline__ void vis_begin(const PhysT<T>& ph, const T* u, VisState<D, T>& s)
 {
-  constexpr int F = D + 2;
-  const T rho = u[0], ri = fr_rcp(rho);
+  s.rho = u[0];
+  s.ri = fr_rcp(u[0]);
 #pragma unroll
-  for (int l = 0; l < D; l++) v[l] = u[l + 1] * ri;
-  T ke = v[0] * v[0];
+  for (int l = 0; l < D; l++) s.v[l] = u[l + 1] * s.ri;
+  s.ke = s.v[0] * s.v[0];
 #pragma unroll
-  for (int l = 1; l < D; l++) ke = fr_fma(v[l], v[l], ke);
-  T inte = fr_fma(T(-0.5), ke, u[F - 1] * ri);
-  T mu, kg;
+  for (int l = 1; l < D; l++) s.ke = fr_fma(s.v[l], s.v[l], s.ke);
+  s.inte = fr_fma(T(-0.5), s.ke, u[D + 1] * s.ri);
   if (ph.fix_vis == T(1)) {
-    mu = ph.mu_inf;
-    kg = ph.kg_inf;
+    s.mu = ph.mu_inf;
+    s.kg = ph.kg_inf;
   } else {
-    T rt = ph.gm1 * inte / ph.rt_inf;
-    mu = ph.mu_inf * fr_pow15<T>(rt) * (T(1) + ph.c_sth) / (rt + ph.c_sth);
-    mu = mu + ph.fix_vis * (ph.mu_inf - mu);
-    kg = mu / ph.prandtl * ph.gamma;
+    T rt = ph.gm1 * s.inte / ph.rt_inf;
+    s.mu = ph.mu_inf * fr_pow15<T>(rt) * (T(1) + ph.c_sth) / (rt + ph.c_sth);
+    s.mu = s.mu + ph.fix_vis * (ph.mu_inf - s.mu);
+    s.kg = s.mu / ph.prandtl * ph.gamma;
   }
-  T dv[D][D];
+}
+template <int D, typename T>
+__device__ __forceinline__ void vis_column(VisState<D, T>& s, int l, const T* g)
+{
 #pragma unroll
-  for (int m = 0; m < D; m++)
+  for (int m = 0; m < D; m++) s.dv[m][l] = fr_fma(-g[0], s.v[m], g[m + 1]) * s.ri;
+  T vdv = s.v[0] * s.dv[0][l];
 #pragma unroll
-    for (int l = 0; l < D; l++) dv[m][l] = fr_fma(-g[0][l], v[m], g[m + 1][l]) * ri;
-  T de[D];
+  for (int m = 1; m < D; m++) vdv = fr_fma(s.v[m], s.dv[m][l], vdv);
+  const T dke = fr_fma(T(0.5) * s.ke, g[0], s.rho * vdv);
+  s.de[l] = fr_fma(-g[0], s.inte, g[D + 1] - dke) * s.ri;
+}
+template <int D, typename T>
+__device__ __forceinline__ void vis_end(const VisState<D, T>& s, T (&tau)[D][D], T (&q)[D])
+{
+  T dsum = s.dv[0][0];
 #pragma unroll
-  for (int l = 0; l < D; l++) {
-    T vdv = v[0] * dv[0][l];
-#pragma unroll
-    for (int m = 1; m < D; m++) vdv = fr_fma(v[m], dv[m][l], vdv);
-    T dke = fr_fma(T(0.5) * ke, g[0][l], rho * vdv);
-    de[l] = fr_fma(-g[0][l], inte, g[F - 1][l] - dke) * ri;
-  }
-  T dsum = dv[0][0];
-#pragma unroll
-  for (int l = 1; l < D; l++) dsum = dsum + dv[l][l];
+  for (int l = 1; l < D; l++) dsum = dsum + s.dv[l][l];
   const T diag = dsum * T(1.0 / 3.0);
-  const T mu2 = T(2) * mu;
+  const T mu2 = T(2) * s.mu;
 #pragma unroll
   for (int m = 0; m < D; m++)
 #pragma unroll
     for (int l = 0; l < D; l++)
-      tau[m][l] = (m == l) ? mu2 * (dv[m][m] - diag) : mu * (dv[m][l] + dv[l][m]);
+      tau[m][l] = (m == l) ? mu2 * (s.dv[m][m] - diag) : s.mu * (s.dv[m][l] + s.dv[l][m]);
 #pragma unroll
-  for (int l = 0; l < D; l++) q[l] = kg * de[l];
+  for (int l = 0; l < D; l++) q[l] = s.kg * s.de[l];
+}
+template <int D, typename T>
+__device__ __forceinline__ void vis_columns(const PhysT<T>& ph, const T* u, T (*g)[D], VisState<D, T>& s)
+{
+  vis_begin<D, T>(ph, u, s);
+#pragma unroll
+  for (int l = 0; l < D; l++) {
+    T c[D + 2];
+#pragma unroll
+    for (int k = 0; k < D + 2; k++) c[k] = g[k][l];
+    vis_column<D, T>(s, l, c);
+  }
 }
 
+// The viscous flux f[k][l] after every column.
 template <int D, typename T>
-__device__ __forceinline__ void vis_flux_fast(const PhysT<T>& ph, const T* u, T (*g)[D], T (*f)[D])
+__device__ __forceinline__ void vis_flux_end(const VisState<D, T>& s, T (*f)[D])
 {
   constexpr int F = D + 2;
-  T v[D], tau[D][D], q[D];
-  vis_core<D, T>(ph, u, g, v, tau, q);
+  T tau[D][D], q[D];
+  vis_end<D, T>(s, tau, q);
 #pragma unroll
   for (int l = 0; l < D; l++) {
     f[0][l] = T(0);
@@ -242,19 +262,19 @@ __device__ __forceinline__ void vis_flux_fast(const PhysT<T>& ph, const T* u, T 
 #pragma unroll
     for (int m = 0; m < D; m++) {
       f[m + 1][l] = -tau[m][l];
-      w = fr_fma(v[m], tau[m][l], w);
+      w = fr_fma(s.v[m], tau[m][l], w);
     }
     f[F - 1][l] = -w;
   }
 }
 
-// The viscous flux projected on n, pr[k - 1] = project(f, k, n) for the
-// components k = 1 .. F-1, without holding all of f.
+// The viscous flux after every column, projected on n: pr[k - 1] =
+// project(f, k, n) for the components k = 1 .. F-1, without holding all of f.
 template <int D, typename T>
-__device__ __forceinline__ void vis_flux_proj(const PhysT<T>& ph, const T* u, T (*g)[D], const T* n, T* pr)
+__device__ __forceinline__ void vis_proj_end(const VisState<D, T>& s, const T* n, T* pr)
 {
-  T v[D], tau[D][D], q[D];
-  vis_core<D, T>(ph, u, g, v, tau, q);
+  T tau[D][D], q[D];
+  vis_end<D, T>(s, tau, q);
 #pragma unroll
   for (int l = 0; l < D; l++) {
     T w = q[l];
@@ -262,11 +282,27 @@ __device__ __forceinline__ void vis_flux_proj(const PhysT<T>& ph, const T* u, T 
     for (int m = 0; m < D; m++) {
       const T fm = -tau[m][l];
       pr[m] = l == 0 ? fm * n[0] : fr_fma(fm, n[l], pr[m]);
-      w = fr_fma(v[m], tau[m][l], w);
+      w = fr_fma(s.v[m], tau[m][l], w);
     }
     const T fe = -w;
     pr[D] = l == 0 ? fe * n[0] : fr_fma(fe, n[l], pr[D]);
   }
+}
+
+template <int D, typename T>
+__device__ __forceinline__ void vis_flux_fast(const PhysT<T>& ph, const T* u, T (*g)[D], T (*f)[D])
+{
+  VisState<D, T> s;
+  vis_columns<D, T>(ph, u, g, s);
+  vis_flux_end<D, T>(s, f);
+}
+
+template <int D, typename T>
+__device__ __forceinline__ void vis_flux_proj(const PhysT<T>& ph, const T* u, T (*g)[D], const T* n, T* pr)
+{
+  VisState<D, T> s;
+  vis_columns<D, T>(ph, u, g, s);
+  vis_proj_end<D, T>(s, n, pr);
 }
 
 // Rusanov common normal flux, static mesh: inters::rusanov_flux,

@@ -34,7 +34,6 @@ struct Bufs {
   int* mate = nullptr;
   unsigned char* side = nullptr;
   double* idetj = nullptr;         // 1/detJ at the solution points (the update multiplies by it)
-  int* err = nullptr;              // set by a kernel whose bounded wait gave up
 };
 
 struct Tile {
@@ -73,24 +72,35 @@ struct Runner {
 };
 
 // Compiled tile variants (elements per CTA, threads per CTA) of the gradient
-// and update kernels per (dims, order); the first entry is the default, the
-// autotuner may pick another.
+// and update kernels per (dims, order); the autotuner may pick any.  The first
+// entry is the default of large meshes, the last one (fewest elements per CTA)
+// that of small ones.  A gradient tile has a thread for each of its F EPB
+// NU / (P+1) line tasks, an update tile one for each of its flux points, in as
+// few idle lanes as whole warps allow.
 template <int DIM, int P> struct Tiles;
 #define FR_TILES(D_, P_, G, U) \
   template <> struct Tiles<D_, P_> { static constexpr Tile grad[] = G; static constexpr Tile upd[] = U; };
 #define T_(...) {__VA_ARGS__}
-FR_TILES(2, 1, T_({32, 128}), T_({32, 128}))
-FR_TILES(2, 2, T_({16, 128}), T_({16, 128}))
-FR_TILES(2, 3, T_({8, 128}, {4, 64}, {16, 256}), T_({8, 128}, {4, 64}, {16, 256}))
-FR_TILES(2, 4, T_({8, 256}), T_({8, 256}))
-FR_TILES(2, 5, T_({4, 160}), T_({4, 160}))
-FR_TILES(3, 1, T_({12, 128}), T_({12, 128}))
-FR_TILES(3, 2, T_({4, 128}, {2, 64}, {8, 256}), T_({4, 128}, {2, 64}, {8, 256}))
-FR_TILES(3, 3, T_({2, 128, 4}, {1, 64, 8}, {2, 192, 2}, {2, 128, 3}, {1, 96, 0}, {4, 256, 2}, {1, 96, 5}, {1, 96, 6},
-                  {1, 64, 8, 1}, {2, 128, 3, 1}, {1, 96, 10}), T_({1, 96, 7}, {1, 64, 8}, {1, 96}, {1, 64}, {2, 128}, {1, 96, 6}, {1, 64, 9}, {2, 192, 3}))
-FR_TILES(3, 4, T_({1, 128}, {1, 160}, {2, 256}), T_({1, 128}, {2, 256}, {1, 160}))
+FR_TILES(2, 1, T_({16, 128, 5}, {4, 32}), T_({16, 128, 4}, {4, 32}))
+FR_TILES(2, 2, T_({10, 128, 5}, {2, 32}), T_({10, 128, 4}, {2, 32}))
+FR_TILES(2, 3, T_({8, 128, 5}, {16, 256, 3}, {2, 32}), T_({8, 128, 4}, {16, 256, 2}, {2, 32}))
+FR_TILES(2, 4, T_({6, 160, 4}, {3, 96, 6}, {1, 32}), T_({5, 128, 5}, {10, 256, 2}, {1, 32}))
+FR_TILES(2, 5, T_({3, 128, 5}, {5, 192, 3}, {1, 64}), T_({3, 128, 5}, {7, 256, 2}, {1, 64}))
+FR_TILES(3, 1, T_({8, 192, 4}, {5, 128, 5}, {1, 32}), T_({8, 192, 3}, {5, 128, 4}, {1, 32}))
+FR_TILES(3, 2, T_({4, 224, 2}, {2, 128, 5}, {1, 64, 10}), T_({4, 224, 3}, {2, 128, 4}, {1, 64, 8}))
+FR_TILES(3, 3, T_({1, 96, 6}, {1, 96, 8}, {1, 96, 5}, {2, 192, 3}, {2, 192, 3, 1}, {1, 96, 7}),
+         T_({1, 96, 6}, {1, 96, 8}, {1, 96, 5}, {2, 192, 3}))
+FR_TILES(3, 4, T_({1, 160, 3}, {1, 160, 4}, {1, 128, 4}), T_({1, 160, 5}, {1, 160, 4}))
 #undef T_
 #undef FR_TILES
+
+// The tile of a mesh before any autotuning: the first, or the last where the
+// first would leave the GPU with fewer than two blocks per SM (148 SMs).
+template <int N>
+int default_tile(const Tile (&t)[N], long long E)
+{
+  return (E + t[0].epb - 1) / t[0].epb >= 296 ? 0 : N - 1;
+}
 
 static void set_smem(const void* k, size_t bytes)
 {
@@ -125,6 +135,8 @@ struct RunnerT : Runner {
       for (int j = 0; j < kMaxN1; j++) L64.D[i][j] = (i <= P && j <= P) ? l.D[i][j] : 0;
     }
     ph = PhysT<TC>::make(p);
+    gsel = default_tile(Tiles<DIM, P>::grad, E);
+    usel = default_tile(Tiles<DIM, P>::upd, E);
   }
   int n_grad_tiles() const override { return NG; }
   int n_update_tiles() const override { return NUP; }
@@ -147,8 +159,8 @@ struct RunnerT : Runner {
     }
     return m;
   }
-  // the bulk-copy kernel folds the interface fluxes into the update (fr_face_update.cuh)
-  static constexpr bool FU = fu_bulk_ok<DIM, P, TC>();
+  // whether the update kernel forms the interface fluxes itself (fr_update.cuh)
+  static constexpr bool FU = update_fused<DIM, P>();
   int launches_per_stage() const override { return FU ? (visc ? 2 : 1) : (visc ? 3 : 2); }
   void set_riemann(int rs) override { riemann = rs; }
   void trace(const Bufs& b, int cur, cudaStream_t s, const double* src = nullptr) override
@@ -166,7 +178,7 @@ struct RunnerT : Runner {
       constexpr int EPB = Tiles<DIM, P>::grad[I].epb, NT = Tiles<DIM, P>::grad[I].nt;
       constexpr int MINB = Tiles<DIM, P>::grad[I].minb > 0 ? Tiles<DIM, P>::grad[I].minb : 1;
       constexpr int PERS = Tiles<DIM, P>::grad[I].pers;
-      constexpr size_t sm = grad_smem_bytes<DIM, P, EPB, TC, LES, grad_alias<DIM, P, EPB, NT, TC, LES, PERS>()>();
+      constexpr size_t sm = grad_smem_bytes<DIM, P, EPB, TC, LES>();
       const void* kfn = (const void*)fr_grad_kernel<DIM, P, EPB, NT, TC, LES, MINB, 1, PERS>;
       static bool once = (set_smem(kfn, sm), true);
       (void)once;
@@ -220,36 +232,26 @@ struct RunnerT : Runner {
     if constexpr (I < NUP) {
       if (I != usel) return update_i<I + 1, VISC, MODE>(b, cur, stage, dt, want_partial, s);
       constexpr int EPB = Tiles<DIM, P>::upd[I].epb, NT = Tiles<DIM, P>::upd[I].nt;
-      if constexpr (FU) {
-        constexpr int MB = Tiles<DIM, P>::upd[I].minb > 0 ? Tiles<DIM, P>::upd[I].minb : 1;
-        if constexpr (DIM == 2) {
-          if (riemann == 2) fu_launch<EPB, NT, VISC, MODE, 2, MB>(b, cur, stage, dt, want_partial, s);
-          else fu_launch<EPB, NT, VISC, MODE, 0, MB>(b, cur, stage, dt, want_partial, s);
-        } else {
-          fu_launch<EPB, NT, VISC, MODE, 0, MB>(b, cur, stage, dt, want_partial, s);
-        }
-      } else {
-        constexpr size_t sm = update_smem_bytes<DIM, P, EPB, NT, VISC, MODE, TC>();
-        static bool once = (set_smem((const void*)fr_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC>, sm), true);
-        (void)once;
-        fr_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC><<<(unsigned)((E + EPB - 1) / EPB), NT, sm, s>>>(
-            b.U, b.REG, (TC*)b.UF[cur ^ 1], (const TC*)b.CF, (const TC*)b.ND, (const TC*)b.DV, (const TC*)b.JG,
-            b.detj64, b.DIV, want_partial ? b.partial : nullptr, E, L, ph, kRK4A[stage], kRK4B[stage], dt,
-            stage == 0 ? 1 : 0);
+      constexpr int MB = Tiles<DIM, P>::upd[I].minb > 0 ? Tiles<DIM, P>::upd[I].minb : 1;
+      if constexpr (FU && DIM == 2) {
+        if (riemann == 2) return upd_launch<EPB, NT, VISC, MODE, 2, MB>(b, cur, stage, dt, want_partial, s);
       }
+      upd_launch<EPB, NT, VISC, MODE, 0, MB>(b, cur, stage, dt, want_partial, s);
     }
   }
   template <int EPB, int NT, int VISC, int MODE, int RS, int MB>
-  void fu_launch(const Bufs& b, int cur, int stage, double dt, bool want_partial, cudaStream_t s)
+  void upd_launch(const Bufs& b, int cur, int stage, double dt, bool want_partial, cudaStream_t s)
   {
-    constexpr size_t sm = face_update_smem_bytes<DIM, P, TC, VISC, MODE, EPB, NT>();
-    const void* kfn = (const void*)fr_face_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC, RS, MB>;
+    constexpr size_t sm = update_smem_bytes<DIM, P, EPB, NT, VISC, MODE, TC>();
+    constexpr int FUSED = FU ? 1 : 0;
+    const void* kfn = (const void*)fr_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC, FUSED, RS, MB>;
     static bool once = (set_smem(kfn, sm), true);
     (void)once;
-    fr_face_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC, RS, MB><<<(unsigned)((E + EPB - 1) / EPB), NT, sm, s>>>(
-        b.U, b.REG, (TC*)b.UF[cur ^ 1], (const TC*)b.UF[cur], b.mate, b.side, (const TC*)b.VF, (const TC*)b.ND,
-        (const TC*)b.DV, (const TC*)b.JG, (const TC*)b.nL, (const TC*)b.tdA, b.idetj, (const TC*)b.BV, b.DIV,
-        want_partial ? b.partial : nullptr, E, L, ph, kRK4A[stage], kRK4B[stage], dt, stage == 0 ? 1 : 0, b.err);
+    fr_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC, FUSED, RS, MB><<<(unsigned)((E + EPB - 1) / EPB), NT, sm, s>>>(
+        b.U, b.REG, (TC*)b.UF[cur ^ 1], (const TC*)b.UF[cur], (const TC*)b.CF, b.mate, b.side, (const TC*)b.VF,
+        (const TC*)b.ND, (const TC*)b.DV, (const TC*)b.JG, (const TC*)b.nL, (const TC*)b.tdA, b.idetj,
+        (const TC*)b.BV, b.DIV, want_partial ? b.partial : nullptr, E, L, ph, kRK4A[stage], kRK4B[stage], dt,
+        stage == 0 ? 1 : 0);
   }
   int merged_args(const Bufs& b, int cur, int stage, double dt, void* gv, void* fv, void* uv) const override
   {
@@ -261,7 +263,7 @@ struct RunnerT : Runner {
           MergedGrad<TC>{b.U, (const TC*)b.UF[cur], b.mate, b.side, (const TC*)b.JG, (const TC*)b.detj,
                          (const TC*)b.nL, (TC*)b.VF, (TC*)b.ND, (TC*)b.DV, (TC*)b.BV, E, nblk, L, ph};
       MergedFace<TC> f{};
-      if constexpr (!merged_fused<P, TC>()) {
+      if constexpr (!FU) {
         const long long n = b.nint + b.nbdy;
         f = MergedFace<TC>{b.face, b.fsign, b.nint, (const TC*)b.UF[cur], (const TC*)b.VF, (const TC*)b.nL,
                            (const TC*)b.tdA, (TC*)b.CF, E * S::NF, b.nbdy, b.bf, b.bt, (const TC*)b.BV,
@@ -271,7 +273,7 @@ struct RunnerT : Runner {
       *static_cast<MergedUpd<TC>*>(uv) =
           MergedUpd<TC>{b.U, b.REG, (TC*)b.UF[cur ^ 1], (const TC*)b.UF[cur], (const TC*)b.CF, b.mate, b.side,
                         (const TC*)b.VF, (const TC*)b.ND, (const TC*)b.DV, (const TC*)b.JG, (const TC*)b.nL,
-                        (const TC*)b.tdA, b.detj64, b.idetj, (const TC*)b.BV, b.DIV, b.err, E, nblk, L, ph,
+                        (const TC*)b.tdA, b.idetj, (const TC*)b.BV, b.DIV, E, nblk, L, ph,
                         kRK4A[stage], kRK4B[stage], dt, stage == 0 ? 1 : 0};
       return P;
     }
