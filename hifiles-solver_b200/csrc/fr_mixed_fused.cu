@@ -207,7 +207,7 @@ fr_status launch_grad(fr_mixed_stage* s, int i, int v, const double* UFc, cudaSt
 {
   const MixedType& t = s->types[i];
   const MixedShape& g = kGradShapes[v];
-  s->kern[i].grad[s->pf][v]<<<blocks_of(t.E, g.epb), g.nth, s->kern[i].smem_a[s->pf][v], st>>>(t, s->fp, UFc,
+  s->kern[i].grad[s->pf][v]<<<blocks_of(t.E, s->kern[i].epb_a[v]), g.nth, s->kern[i].smem_a[s->pf][v], st>>>(t, s->fp, UFc,
                                                                                                  s->ph);
   return mlaunched("mixed_grad_kernel");
 }
@@ -222,7 +222,7 @@ fr_status launch_upd(fr_mixed_stage* s, int i, int v, int mode, int stage, doubl
   t.partial = norms ? s->partials[i] : nullptr;
   const MixedShape& u = kUpdShapes[v];
   auto k = mode ? s->kern[i].upd1[s->pf][v] : s->kern[i].upd0[s->pf][v];
-  k<<<blocks_of(t.E, u.epb), u.nth, s->kern[i].smem_b[v], st>>>(t, s->fp, UFc, UFn, s->ph, A[stage], B[stage], dt);
+  k<<<blocks_of(t.E, s->kern[i].epb_b[v]), u.nth, s->kern[i].smem_b[v], st>>>(t, s->fp, UFc, UFn, s->ph, A[stage], B[stage], dt);
   return mlaunched("mixed_update_kernel");
 }
 
@@ -258,7 +258,7 @@ fr_status launch_trace(fr_mixed_stage* s, cudaStream_t st)
 {
   return for_types(s, st, [&](int i, cudaStream_t q) {
     const MixedType& t = s->types[i];
-    s->kern[i].trace<<<blocks_of(t.E, kMixedEPB), kMixedNT, s->kern[i].smem_c, q>>>(t, s->NT, s->UF[s->cur]);
+    s->kern[i].trace<<<blocks_of(t.E, s->kern[i].epb_c), kMixedNT, s->kern[i].smem_c, q>>>(t, s->NT, s->UF[s->cur]);
     return mlaunched("mixed_trace_kernel");
   });
 }
@@ -639,7 +639,7 @@ fr_status fr_mixed_stage_advance_norms(fr_mixed_stage* s, int n_steps, double dt
   double n_upts = 0.0;
   for (int i = 0; i < s->n_types; i++) {
     np.p[i] = s->partials[i];
-    np.nb[i] = s->types[i].E > 0 ? (int)blocks_of(s->types[i].E, kUpdShapes[s->uv[i]].epb) : 0;
+    np.nb[i] = s->types[i].E > 0 ? (int)blocks_of(s->types[i].E, s->kern[i].epb_b[s->uv[i]]) : 0;
     n_upts += (double)s->types[i].NU * (double)s->types[i].E;
   }
   mixed_norm_finalize<<<s->F, kNormThreads, 0, st>>>(np, s->n_types, s->F, n_upts, s->norms_dev);

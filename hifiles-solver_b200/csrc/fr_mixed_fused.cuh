@@ -45,36 +45,26 @@ struct MPlan {
   static constexpr int KS_U = c4(NU) / 4, KS_F = c4(NF) / 4, KS_T = c4(D * NU) / 4;
   static constexpr int NTL = NP / 8, NTLG = NGP / 8;
   static constexpr int TN = tiles_per_unit(NTL), TNG = tiles_per_unit(NTLG);
-  // kernel A: the matrices U | own traces | gradient (the neighbours' traces
-  // [F][EF] before it) | X (delta, then the gradient at the flux points, then
-  // the transformed flux); then what the load phase stages: left normals
-  // [D][EF], detJ [EU], JGinv [EPB][DD NU] (when it fits), mate and side [EF]
-  // ints each
+  // kernel A: the matrices U | own traces | gradient | X (delta, then the
+  // gradient at the flux points, then the transformed flux); then what else the
+  // load phase stages: left normals [D][EF], detJ [EU], JGinv [EPB][DD NU] (when
+  // it fits)
   static constexpr int oU = 0, oUF = oU + NP * ldU, oG = oUF + NP * ldF, oX = oG + NP * ldG;
   static constexpr int nX = cmax(cmax(NP * ldF, NGP * ldF), NP * ldT);
   static constexpr int oNL = oX + r2(nX), oDJ = oNL + r2(D * EF), oJG = oDJ + r2(EU);
   // JGinv is staged when MINB blocks with it fit in an SM's shared memory
   // (228 KB, 1 KB reserved per block), else read through the L1 cache
-  static constexpr bool SJ = (size_t)MINB * (sizeof(double) * (size_t)(oJG + r2(DD * EU) + r2(EF)) + 1024) <=
-                                 228 * 1024 &&
-                             sizeof(double) * (size_t)(oJG + r2(DD * EU) + r2(EF)) <= kMixedSmemMax;
-  static constexpr int oIA = oJG + (SJ ? r2(DD * EU) : 0);
-  static constexpr int nA = oIA + r2(EF);
-  // kernel B: the jump norm_tconf - norm_tdisf (norm_tdisf first) | own traces
-  // [F][EF] (the new state [NP][ldU] after the flux phase) | neighbours'
-  // traces | own and neighbours' viscous projections [F-1][EF] | left normals
-  // [D][EF] | tdA [EF] | div_tdisf, RK register, state [F][EU] | detJ [EU] |
-  // mate and side
-  static constexpr int oJ = 0, oUo = r2(NP * ldF), oUN = oUo + r2(cmax(F * EF, NP * ldU));
-  static constexpr int oVo = oUN + r2(F * EF), oVN = oVo + r2((F - 1) * EF), oNLb = oVN + r2((F - 1) * EF);
-  static constexpr int oTA = oNLb + r2(D * EF), oDV = oTA + r2(EF), oRG = oDV + r2(F * EU), oUO = oRG + r2(F * EU);
-  static constexpr int oDJb = oUO + r2(F * EU), oIB = oDJb + r2(EU);
-  static constexpr int nB = oIB + r2(EF);
+  static constexpr bool SJ = (size_t)MINB * (sizeof(double) * (size_t)(oJG + r2(DD * EU)) + 1024) <= 228 * 1024 &&
+                             sizeof(double) * (size_t)(oJG + r2(DD * EU)) <= kMixedSmemMax;
+  static constexpr int nA = oJG + (SJ ? r2(DD * EU) : 0);
+  // kernel B: the jump norm_tconf - norm_tdisf | the new state [NP][ldU] |
+  // div_tdisf, RK register (then |div/detJ| for residual norms), state [F][EU] |
+  // detJ [EU]
+  static constexpr int oJ = 0, oUn = r2(NP * ldF), oDV = oUn + r2(NP * ldU), oRG = oDV + r2(F * EU);
+  static constexpr int oUO = oRG + r2(F * EU), oDJb = oUO + r2(F * EU), nB = oDJb + r2(EU);
   // trace kernel: the state
   static constexpr int nC = NP * ldU;
   static_assert(ldT >= c4(D * NU) && ldG >= c8(D * NU) && ldF >= c8(NF) && ldU >= c4(NU), "plan");
-  static_assert(F * EF <= NP * ldG, "the neighbours' traces fit in the gradient's place");
-  static_assert(F * EU <= oNLb - oUN, "residual terms fit in the neighbours' traces and projections");
 };
 
 struct MixedType {
@@ -208,24 +198,36 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, Mixe
   double* sUF = msm + Q::oUF;
   double* sG = msm + Q::oG;
   double* sX = msm + Q::oX;
-  double* sUN = sG;  // neighbours' traces, until the gradient product
   double* sNL = msm + Q::oNL;
   double* sDJ = msm + Q::oDJ;
   double* sJG = msm + Q::oJG;
-  int* sMate = reinterpret_cast<int*>(msm + Q::oIA);
-  int* sSide = sMate + EF;
   const int tid = threadIdx.x, warp = tid >> 5;
   const long long E = t.E, NT = m.NT, e0 = (long long)blockIdx.x * EPB;
   const int nval = (int)(E - e0 < EPB ? E - e0 : EPB), nuv = nval * NU, nfv = nval * NF;
   const long long gb = t.off + (long long)NF * e0;
 
-  // load phase: asynchronous copies (cp.async), many in flight per thread;
-  // first everything at known addresses, then the neighbours' traces through
-  // the staged mate.  The matrices are not cleared: only the padding rows
-  // the products read are zeroed (U here, delta and the flux before their
-  // products); every other padding entry only reaches outputs that are not
+  // load phase: asynchronous copies (cp.async), many in flight per thread, of
+  // everything at known addresses; the neighbours' traces go straight to the
+  // registers of the threads that use them (up to four flux points per thread:
+  // first every mate, then every trace, so two round trips and no barrier; a
+  // boundary point reads its own, unused).  The matrices are not cleared: only the
+  // padding rows the products read are zeroed (U and delta here, the flux before
+  // its products); every other padding entry only reaches outputs that are not
   // written.
+  constexpr int IT = (EF + NTH - 1) / NTH;
+  constexpr bool PRE = IT <= 4;
+  int mtr[PRE ? IT : 1], sdr[PRE ? IT : 1];
+  if constexpr (PRE) {
+#pragma unroll
+    for (int it = 0; it < IT; it++) {
+      const int r = tid + it * NTH;
+      const long long g = gb + (r < nfv ? r : 0);
+      mtr[it] = m.mate[g];
+      sdr[it] = m.side[g];
+    }
+  }
   zero_pad_rows<NU, c4(NU), Q::ldU, Q::NP, NTH>(sU);
+  zero_pad_rows<NF, c4(NF), Q::ldF, Q::NP, NTH>(sX);  // delta's padding rows
   load_state<F, NU, EPB, Q::ldU, NTH>(sU, t.U, e0, E, nval);
   for (int r = tid; r < nfv; r += NTH) {
     const int el = r / NF, f = r - el * NF;
@@ -235,8 +237,6 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, Mixe
     for (int k = 0; k < F; k++) cp_async<8>(dst + k * Q::ldF, UFc + g + NT * k);
 #pragma unroll
     for (int d = 0; d < D; d++) cp_async<8>(&sNL[d * EF + r], m.nL + g + NT * d);
-    cp_async<4>(&sMate[r], m.mate + g);
-    cp_async<4>(&sSide[r], m.side + g);
   }
   for (int i = tid; i < nuv; i += NTH) {
     cp_async<8>(&sDJ[i], t.detj + (size_t)NU * e0 + i);
@@ -244,23 +244,32 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, Mixe
 #pragma unroll
       for (int q = 0; q < DD; q++) cp_async<8>(&sJG[i + q * nuv], t.JG + (size_t)DD * NU * e0 + i + q * nuv);
   }
-  cp_async_wait_all();
-  __syncthreads();
-  for (int r = tid; r < nfv; r += NTH) {
-    const int mt = sMate[r];
-    if (mt < 0) continue;
+  double unr[PRE ? IT : 1][F];
+  auto gather = [&](int r, int mt, double (&un)[F]) {
+    const long long h = mt < 0 ? gb + (r < nfv ? r : 0) : (long long)mt;
 #pragma unroll
-    for (int k = 0; k < F; k++) cp_async<8>(&sUN[k * EF + r], UFc + mt + NT * k);
+    for (int k = 0; k < F; k++) un[k] = UFc[h + NT * k];
+  };
+  if constexpr (PRE) {
+#pragma unroll
+    for (int it = 0; it < IT; it++) gather(tid + it * NTH, mtr[it], unr[it]);
   }
-  zero_pad_rows<NF, c4(NF), Q::ldF, Q::NP, NTH>(sX);  // delta's padding rows
   cp_async_wait_all();
   __syncthreads();
   auto jg = [&](int i) { return Q::SJ ? sJG + DD * i : t.JG + (size_t)DD * ((size_t)NU * e0 + i); };
 
   // LDG common solution at the own flux points: delta = u_c - u_own into X
-  for (int i = tid; i < nfv; i += NTH) {
-    const int el = i / NF, f = i - el * NF;
-    const int sd = sSide[i];
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const int i = tid + it * NTH;
+    if (i >= nfv) continue;
+    const int el = i / NF, f = i - el * NF, pi = PRE ? it : 0;
+    if constexpr (!PRE) {
+      mtr[0] = m.mate[gb + i];
+      sdr[0] = m.side[gb + i];
+      gather(i, mtr[0], unr[0]);
+    }
+    const int sd = sdr[pi];
     double n[D], uo[F];
 #pragma unroll
     for (int d = 0; d < D; d++) n[d] = sNL[d * EF + i];
@@ -279,7 +288,7 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, Mixe
       const double pen = ldg_beta<D, double>(ph.pen_fact, n);
 #pragma unroll
       for (int k = 0; k < F; k++) {
-        const double un = sUN[k * EF + i];
+        const double un = unr[pi][k];
         const double ul = left ? uo[k] : un, ur = left ? un : uo[k];
         const double uc = 0.5 * (ul + ur) - pen * (ul - ur);
         dx[k * Q::ldF] = uc - uo[k];
@@ -346,10 +355,13 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, Mixe
   __syncthreads();
 
   // viscous normal projections (interior points) and boundary viscous fluxes
-  for (int i = tid; i < nfv; i += NTH) {
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const int i = tid + it * NTH;
+    if (i >= nfv) continue;
     const int el = i / NF, f = i - el * NF;
     const long long g = gb + i;
-    const int mt = sMate[i], sd = sSide[i];
+    const int sd = PRE ? sdr[PRE ? it : 0] : m.side[g];
     double n[D], uo[F], gf[F][D];
 #pragma unroll
     for (int d = 0; d < D; d++) n[d] = sNL[d * EF + i];
@@ -369,7 +381,7 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, Mixe
       }
 #pragma unroll
       for (int d = 0; d < D; d++) q.n[d] = n[d];
-      vis_boundary<D, double, false>(ph, sd >> 2, q, m.BV + (size_t)(-1 - (long long)mt) * F);
+      vis_boundary<D, double, false>(ph, sd >> 2, q, m.BV + (size_t)(-1 - (long long)m.mate[g]) * F);
     } else {
       double pr[F - 1];
       vis_flux_proj<D, double>(ph, uo, gf, n, pr);
@@ -519,8 +531,20 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_inv_kernel(MixedType t, Mixed
 
 // ------------------------------------------------------------------ kernel B
 // MODE 1: RK45 stage update (rk_a, rk_b, dt) and the new traces into UFn;
-// MODE 0: div_tconf_upts into t.DIV only.  Like kernel A, a load phase first
-// stages every global read of the block in shared memory.
+// MODE 0: div_tconf_upts into t.DIV only.  A flux point's inputs (own and
+// neighbour's trace and projections, normal flux, normal, dA) are each used
+// once, by its own thread: they go to registers, the neighbour's as soon as the
+// mate has arrived; what the product's epilogue needs (divergence, register,
+// state, detJ) is copied to shared memory meanwhile.  Staging all of it in
+// shared memory took two rounds of copies with a barrier each and twice the
+// shared memory per element.
+template <int D, int VISC>
+struct FptRegs {
+  static constexpr int F = D + 2;
+  int mt, sd;
+  double uo[F], un[F], nd[F], vo[VISC ? F - 1 : 1], vn[VISC ? F - 1 : 1], n[D], tl;
+};
+
 template <int D, int NU, int NF, int EPB, int NTH, int MINB, int MODE, int VISC = 1, int RIEMANN = 0>
 __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, MixedFpts m,
                                                                  const double* __restrict__ UFc,
@@ -528,50 +552,47 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, Mi
                                                                  double rk_a, double rk_b, double dt)
 {
   using Q = MPlan<D, NU, NF, EPB>;
-  constexpr int F = D + 2, NW = NTH / 32, EU = Q::EU, EF = Q::EF;
+  constexpr int F = D + 2, NW = NTH / 32, EU = Q::EU, EF = Q::EF, IT = (EF + NTH - 1) / NTH;
   extern __shared__ __align__(16) double msm[];
   double* sJ = msm + Q::oJ;
-  double* sUo = msm + Q::oUo;
-  double* sUn = sUo;  // the new state, after the flux phase
-  double* sUN = msm + Q::oUN;
-  double* sRes = sUN;  // |div/detJ| [F][EU] for residual norms, after the flux phase
-  double* sVo = msm + Q::oVo;
-  double* sVN = msm + Q::oVN;
-  double* sNL = msm + Q::oNLb;
-  double* sTA = msm + Q::oTA;
+  double* sUn = msm + Q::oUn;
   double* sDV = msm + Q::oDV;
   double* sRG = msm + Q::oRG;
+  double* sRes = sRG;  // |div/detJ| [F][EU] for residual norms: each entry by the thread that read the register
   double* sUO = msm + Q::oUO;
   double* sDJ = msm + Q::oDJb;
-  int* sMate = reinterpret_cast<int*>(msm + Q::oIB);
-  int* sSide = sMate + EF;
   const int tid = threadIdx.x, warp = tid >> 5;
   const long long E = t.E, NT = m.NT, e0 = (long long)blockIdx.x * EPB;
   const int nval = (int)(E - e0 < EPB ? E - e0 : EPB), nuv = nval * NU, nfv = nval * NF;
   const long long gb = t.off + (long long)NF * e0;
   const size_t NFE = (size_t)NF * E, NUE = (size_t)NU * E;
 
-  // load phase: asynchronous copies, as in the gradient kernel
-  zero_pad_rows<NF, c4(NF), Q::ldF, Q::NP, NTH>(sJ);
-  for (int r = tid; r < nfv; r += NTH) {
-    const int el = r / NF, f = r - el * NF;
+  auto load = [&](int r, FptRegs<D, VISC>& q) {
     const long long g = gb + r;
-    double* dj = sJ + el * F * Q::ldF + f;
+    q.mt = m.mate[g];
+    q.sd = m.side[g];
     const double* nd = t.ND + (size_t)NF * e0 + r;
 #pragma unroll
     for (int k = 0; k < F; k++) {
-      cp_async<8>(&sUo[k * EF + r], UFc + g + NT * k);
-      cp_async<8>(dj + k * Q::ldF, nd + NFE * k);
+      q.uo[k] = UFc[g + NT * k];
+      q.nd[k] = nd[NFE * k];
     }
-    if constexpr (VISC != 0)
+    if constexpr (VISC != 0) {
 #pragma unroll
-      for (int k = 0; k < F - 1; k++) cp_async<8>(&sVo[k * EF + r], m.VF + g + NT * k);
+      for (int k = 0; k < F - 1; k++) q.vo[k] = m.VF[g + NT * k];
+    }
 #pragma unroll
-    for (int d = 0; d < D; d++) cp_async<8>(&sNL[d * EF + r], m.nL + g + NT * d);
-    cp_async<4>(&sMate[r], m.mate + g);
-    cp_async<4>(&sSide[r], m.side + g);
-    cp_async<8>(&sTA[r], m.tdA + g);
-  }
+    for (int d = 0; d < D; d++) q.n[d] = m.nL[g + NT * d];
+    q.tl = m.tdA[g];
+    // the neighbour's values (a boundary point reads its own, unused), no branch between the loads
+    const long long h = q.mt < 0 ? g : (long long)q.mt;
+#pragma unroll
+    for (int k = 0; k < F; k++) q.un[k] = UFc[h + NT * k];
+    if constexpr (VISC != 0) {
+#pragma unroll
+      for (int k = 0; k < F - 1; k++) q.vn[k] = m.VF[h + NT * k];
+    }
+  };
   for (int r = tid; r < nuv; r += NTH) {
     const size_t ix = (size_t)NU * e0 + r;
 #pragma unroll
@@ -584,73 +605,57 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, Mi
     }
     if (MODE == 1) cp_async<8>(&sDJ[r], t.detj + ix);
   }
-  cp_async_wait_all();
-  __syncthreads();
-  for (int r = tid; r < nfv; r += NTH) {
-    const int mt = sMate[r];
-    if (mt < 0) continue;
-#pragma unroll
-    for (int k = 0; k < F; k++) cp_async<8>(&sUN[k * EF + r], UFc + mt + NT * k);
-    if constexpr (VISC != 0)
-#pragma unroll
-      for (int k = 0; k < F - 1; k++) cp_async<8>(&sVN[k * EF + r], m.VF + mt + NT * k);
-  }
-  cp_async_wait_all();
-  __syncthreads();
+  zero_pad_rows<NF, c4(NF), Q::ldF, Q::NP, NTH>(sJ);
 
   // common normal fluxes times the own tdA, minus norm_tdisf
-  for (int i = tid; i < nfv; i += NTH) {
+#pragma unroll
+  for (int it = 0; it < IT; it++) {
+    const int i = tid + it * NTH;
+    if (i >= nfv) continue;
+    FptRegs<D, VISC> q;
+    load(i, q);
     const int el = i / NF, f = i - el * NF;
-    const int mt = sMate[i], sd = sSide[i];
-    double n[D], uo[F], c[F];
-#pragma unroll
-    for (int d = 0; d < D; d++) n[d] = sNL[d * EF + i];
-#pragma unroll
-    for (int k = 0; k < F; k++) uo[k] = sUo[k * EF + i];
-    const double tl = sTA[i];
-    if (sd >> 2) {
-      FUBdy<D, double> q;
+    double c[F];
+    if (q.sd >> 2) {
+      FUBdy<D, double> b;
 #pragma unroll
       for (int k = 0; k < F; k++) {
-        q.ul[k] = uo[k];
-        q.bv[k] = VISC ? m.BV[(size_t)(-1 - (long long)mt) * F + k] : 0.0;
+        b.ul[k] = q.uo[k];
+        b.bv[k] = VISC ? m.BV[(size_t)(-1 - (long long)q.mt) * F + k] : 0.0;
       }
 #pragma unroll
-      for (int d = 0; d < D; d++) q.n[d] = n[d];
-      q.tl = tl;
-      fu_boundary<D, VISC, double, RIEMANN>(ph, sd >> 2, q, c, 1);
+      for (int d = 0; d < D; d++) b.n[d] = q.n[d];
+      b.tl = q.tl;
+      fu_boundary<D, VISC, double, RIEMANN>(ph, q.sd >> 2, b, c, 1);
     } else {
-      const bool left = sd & 1;
+      const bool left = q.sd & 1;
       double ul[F], ur[F], fn[F];
 #pragma unroll
       for (int k = 0; k < F; k++) {
-        const double v = sUN[k * EF + i];
-        ul[k] = left ? uo[k] : v;
-        ur[k] = left ? v : uo[k];
+        ul[k] = left ? q.uo[k] : q.un[k];
+        ur[k] = left ? q.un[k] : q.uo[k];
       }
-      if constexpr (RIEMANN == 2 && D == 2) roe<double>(ph, ul, ur, n, fn);
-      else rusanov<D, double>(ph, ul, ur, n, fn);
+      if constexpr (RIEMANN == 2 && D == 2) roe<double>(ph, ul, ur, q.n, fn);
+      else rusanov<D, double>(ph, ul, ur, q.n, fn);
 #pragma unroll
-      for (int k = 0; k < F; k++) c[k] = left ? fn[k] * tl : -fn[k] * tl;
+      for (int k = 0; k < F; k++) c[k] = left ? fn[k] * q.tl : -fn[k] * q.tl;
       if constexpr (VISC != 0) {
-        double nn = n[0] * n[0];
+        double nn = q.n[0] * q.n[0];
 #pragma unroll
-        for (int d = 1; d < D; d++) nn = fma(n[d], n[d], nn);
-        const double pen = ldg_beta<D, double>(ph.pen_fact, n);
+        for (int d = 1; d < D; d++) nn = fma(q.n[d], q.n[d], nn);
+        const double pen = ldg_beta<D, double>(ph.pen_fact, q.n);
 #pragma unroll
         for (int k = 0; k < F; k++) {
-          const double ao = k ? sVo[(k - 1) * EF + i] : 0.0, an = k ? sVN[(k - 1) * EF + i] : 0.0;
+          const double ao = k ? q.vo[k ? k - 1 : 0] : 0.0, an = k ? q.vn[k ? k - 1 : 0] : 0.0;
           const double fv = ldg_normal<double>(left ? ao : an, left ? an : ao, ul[k], ur[k], pen, ph.tau, nn);
-          c[k] = left ? c[k] + fv * tl : c[k] + (-fv) * tl;
+          c[k] = left ? c[k] + fv * q.tl : c[k] + (-fv) * q.tl;
         }
       }
     }
 #pragma unroll
-    for (int k = 0; k < F; k++) {
-      double* p = sJ + (el * F + k) * Q::ldF + f;
-      *p = c[k] - *p;
-    }
+    for (int k = 0; k < F; k++) sJ[(el * F + k) * Q::ldF + f] = c[k] - q.nd[k];
   }
+  cp_async_wait_all();
   __syncthreads();
 
   // div_tconf = div_tdisf + opp_3 jump, then the RK45 update
@@ -671,10 +676,10 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, Mi
       if (MODE == 0) {
         t.DIV[ix] = div;
       } else {
-        // |div/detJ - const_src - src| of compute_res_upts (src/eles.cpp:6086-6115)
-        if (t.partial) sRes[li] = fabs(div / sDJ[el * NU + r] - 0.0 - 0.0);
-        const double rhs = -div / sDJ[el * NU + r] + 0.0 + 0.0;
+        const double rhs = -div / sDJ[el * NU + r];
         const double res = fma(rk_a, sRG[li], dt * rhs);
+        // |div/detJ| of compute_res_upts (src/eles.cpp:6086-6115; no sources here)
+        if (t.partial) sRes[li] = fabs(rhs);
         t.REG[ix] = res;
         const double un = fma(rk_b, res, sUO[li]);
         t.U[ix] = un;
@@ -754,10 +759,18 @@ __global__ void __launch_bounds__(NTH) mixed_trace_kernel(MixedType t, long long
 struct MixedShape {
   int epb, nth, minb;
 };
-constexpr MixedShape kGradShapes[] = {{8, 256, 1}, {4, 128, 3}, {8, 128, 2}, {4, 128, 4}, {8, 256, 2}};
-constexpr MixedShape kUpdShapes[] = {{8, 256, 2}, {4, 128, 4}, {8, 128, 4}};
+constexpr MixedShape kGradShapes[] = {{8, 256, 1}, {4, 128, 3}, {4, 160, 3}, {4, 128, 4}, {8, 256, 2}};
+constexpr MixedShape kUpdShapes[] = {{8, 256, 2}, {4, 160, 3}, {4, 128, 4}};
 constexpr int kNGrad = sizeof(kGradShapes) / sizeof(kGradShapes[0]);
 constexpr int kNUpd = sizeof(kUpdShapes) / sizeof(kUpdShapes[0]);
+// Elements per block of a type with NF flux points: the shape's, or as many
+// (in fours, whole column tiles) as give each flux point a thread.  Types with
+// few points would leave most of a block idle otherwise: triangles of P = 2 had
+// 36 flux points on 128 threads (update kernel of 17280: 26.5 us).
+__host__ __device__ constexpr int shape_epb(MixedShape s, int nf)
+{
+  return cmax(s.epb, s.nth / nf / 4 * 4);
+}
 
 using GradFn = void (*)(MixedType, MixedFpts, const double*, PhysT<double>);
 using UpdFn = void (*)(MixedType, MixedFpts, const double*, double*, PhysT<double>, double, double, double);
@@ -770,6 +783,7 @@ constexpr int kNForms = 3;
 
 struct MixedKernels {
   int D, NU, NF;
+  int epb_a[kNGrad], epb_b[kNUpd], epb_c;  // elements per block of each launch shape
   GradFn grad[kNForms][kNGrad];
   size_t smem_a[kNForms][kNGrad];
   UpdFn upd0[kNForms][kNUpd], upd1[kNForms][kNUpd];
@@ -782,35 +796,40 @@ template <int D, int NU, int NF, int V>
 void fill_grad(MixedKernels& k)
 {
   constexpr MixedShape g = kGradShapes[V];
-  k.smem_a[0][V] = sizeof(double) * MPlan<D, NU, NF, g.epb, g.minb>::nA;
-  k.grad[0][V] = k.smem_a[0][V] <= kMixedSmemMax ? mixed_grad_kernel<D, NU, NF, g.epb, g.nth, g.minb> : nullptr;
+  constexpr int epb = shape_epb(g, NF);
+  k.epb_a[V] = epb;
+  k.smem_a[0][V] = sizeof(double) * MPlan<D, NU, NF, epb, g.minb>::nA;
+  k.grad[0][V] = k.smem_a[0][V] <= kMixedSmemMax ? mixed_grad_kernel<D, NU, NF, epb, g.nth, g.minb> : nullptr;
 }
 
 template <int D, int NU, int NF, int V>
 void fill_upd(MixedKernels& k)
 {
   constexpr MixedShape u = kUpdShapes[V];
-  k.smem_b[V] = sizeof(double) * MPlan<D, NU, NF, u.epb>::nB;
+  constexpr int epb = shape_epb(u, NF);
+  k.epb_b[V] = epb;
+  k.smem_b[V] = sizeof(double) * MPlan<D, NU, NF, epb>::nB;
   const bool fits = k.smem_b[V] <= kMixedSmemMax;
-  k.upd0[0][V] = fits ? mixed_update_kernel<D, NU, NF, u.epb, u.nth, u.minb, 0> : nullptr;
-  k.upd1[0][V] = fits ? mixed_update_kernel<D, NU, NF, u.epb, u.nth, u.minb, 1> : nullptr;
+  k.upd0[0][V] = fits ? mixed_update_kernel<D, NU, NF, epb, u.nth, u.minb, 0> : nullptr;
+  k.upd1[0][V] = fits ? mixed_update_kernel<D, NU, NF, epb, u.nth, u.minb, 1> : nullptr;
 }
 
 template <int D, int NU, int NF>
 void fill_euler(MixedKernels& k)
 {
   constexpr MixedShape g = kGradShapes[1], u = kUpdShapes[1];
-  const size_t sa = sizeof(double) * MPlanInv<D, NU, NF, g.epb>::nI;
+  constexpr int ge = shape_epb(g, NF), ue = shape_epb(u, NF);
+  const size_t sa = sizeof(double) * MPlanInv<D, NU, NF, ge>::nI;
   const bool fa = sa <= kMixedSmemMax, fb = k.smem_b[1] <= kMixedSmemMax;
   for (int f = 1; f < kNForms; f++) {
     k.smem_a[f][1] = sa;
-    k.grad[f][1] = fa ? mixed_inv_kernel<D, NU, NF, g.epb, g.nth, g.minb> : nullptr;
+    k.grad[f][1] = fa ? mixed_inv_kernel<D, NU, NF, ge, g.nth, g.minb> : nullptr;
   }
-  k.upd0[1][1] = fb ? mixed_update_kernel<D, NU, NF, u.epb, u.nth, u.minb, 0, 0, 0> : nullptr;
-  k.upd1[1][1] = fb ? mixed_update_kernel<D, NU, NF, u.epb, u.nth, u.minb, 1, 0, 0> : nullptr;
+  k.upd0[1][1] = fb ? mixed_update_kernel<D, NU, NF, ue, u.nth, u.minb, 0, 0, 0> : nullptr;
+  k.upd1[1][1] = fb ? mixed_update_kernel<D, NU, NF, ue, u.nth, u.minb, 1, 0, 0> : nullptr;
   if constexpr (D == 2) {
-    k.upd0[2][1] = fb ? mixed_update_kernel<D, NU, NF, u.epb, u.nth, u.minb, 0, 0, 2> : nullptr;
-    k.upd1[2][1] = fb ? mixed_update_kernel<D, NU, NF, u.epb, u.nth, u.minb, 1, 0, 2> : nullptr;
+    k.upd0[2][1] = fb ? mixed_update_kernel<D, NU, NF, ue, u.nth, u.minb, 0, 0, 2> : nullptr;
+    k.upd1[2][1] = fb ? mixed_update_kernel<D, NU, NF, ue, u.nth, u.minb, 1, 0, 2> : nullptr;
   }
 }
 
@@ -831,8 +850,10 @@ MixedKernels mixed_kernels()
   fill_upd<D, NU, NF, 2>(k);
   static_assert(kNGrad == 5 && kNUpd == 3, "one fill per shape");
   fill_euler<D, NU, NF>(k);
-  k.trace = mixed_trace_kernel<D, NU, NF, kMixedEPB, kMixedNT>;
-  k.smem_c = sizeof(double) * MPlan<D, NU, NF, kMixedEPB>::nC;
+  constexpr int te = shape_epb(MixedShape{kMixedEPB, kMixedNT, 1}, NF);
+  k.epb_c = te;
+  k.trace = mixed_trace_kernel<D, NU, NF, te, kMixedNT>;
+  k.smem_c = sizeof(double) * MPlan<D, NU, NF, te>::nC;
   return k;
 }
 
