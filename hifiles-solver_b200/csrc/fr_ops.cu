@@ -152,7 +152,7 @@ dense_apply_kernel(int m, int k, long long ncols, int nd, OpSet ops, const doubl
 }
 
 // FP64 tensor-core form of the same products (mma.sync m8n8k4 f64): a block
-// stages a tile of 64-512 columns (the widest within 100 kB) of every B_d in
+// stages a tile of 32-512 columns (the widest within 100 kB) of every B_d in
 // shared memory by asynchronous copies (column-major,
 // leading dimension ldk = 4 or 12 mod 16 doubles, rows k .. ceil4(k) zeroed),
 // and each warp unit computes 8 rows x 32 columns: the accumulator starts at
@@ -268,20 +268,23 @@ fr_status dense_mma_launch(int m, int k, long long ncols, int nd, const OpSet& o
   const int ldk = mma_ld(k), nb = fan ? 1 : nd;
   // the widest column tile within 100 kB (short operators get wide tiles, so
   // a block's staging is spread over enough products), narrowed while the
-  // grid would not give every SM two blocks
+  // grid would not give every SM four blocks: with two, whole blocks left over
+  // idle a third of the GPU (16^3 hexes of P = 3, 20480 columns: 320 blocks of
+  // 64 columns are 2.2 per SM)
   int nct = 64;
   for (int c : {512, 256, 128})
     if (mma_smem(k, nb, c) <= 100 * 1024) {
       nct = c;
       break;
     }
-  while (nct > 64 && (ncols + nct - 1) / nct < 2 * 148) nct /= 2;
+  while (nct > 32 && (ncols + nct - 1) / nct < 4 * 148) nct /= 2;
   const size_t smem = mma_smem(k, nb, nct);
   auto pick = [&](auto kt, auto kf) { return fan ? kt : kf; };
   auto kern = nct == 512   ? pick(dense_mma_kernel<true, 512>, dense_mma_kernel<false, 512>)
               : nct == 256 ? pick(dense_mma_kernel<true, 256>, dense_mma_kernel<false, 256>)
               : nct == 128 ? pick(dense_mma_kernel<true, 128>, dense_mma_kernel<false, 128>)
-                           : pick(dense_mma_kernel<true, 64>, dense_mma_kernel<false, 64>);
+              : nct == 64  ? pick(dense_mma_kernel<true, 64>, dense_mma_kernel<false, 64>)
+                           : pick(dense_mma_kernel<true, 32>, dense_mma_kernel<false, 32>);
   // every instantiation may use up to 100 kB: set once per device
   static unsigned long long attr_set = 0;
   int dev = 0;
@@ -290,7 +293,8 @@ fr_status dense_mma_launch(int m, int k, long long ncols, int nd, const OpSet& o
     const void* all[] = {(const void*)dense_mma_kernel<true, 512>, (const void*)dense_mma_kernel<false, 512>,
                          (const void*)dense_mma_kernel<true, 256>, (const void*)dense_mma_kernel<false, 256>,
                          (const void*)dense_mma_kernel<true, 128>, (const void*)dense_mma_kernel<false, 128>,
-                         (const void*)dense_mma_kernel<true, 64>, (const void*)dense_mma_kernel<false, 64>};
+                         (const void*)dense_mma_kernel<true, 64>, (const void*)dense_mma_kernel<false, 64>,
+                         (const void*)dense_mma_kernel<true, 32>, (const void*)dense_mma_kernel<false, 32>};
     for (const void* f : all) {
       cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       if (e != cudaSuccess) return op_fail(FR_ERR_CUDA, cudaGetErrorString(e));
@@ -492,7 +496,7 @@ __global__ void vis_flux_kernel(int nu, long long E, const double* __restrict__ 
 #pragma unroll
     for (int d = 0; d < D; d++) g[k][d] = GU[i + NE * (k + (size_t)F * d)];
   }
-  vis_flux<D, double>(ph, q, g, f);
+  vis_flux_fast<D, double>(ph, q, g, f);
   const double* G = JG + (size_t)D * D * i;
 #pragma unroll
   for (int k = 0; k < F; k++)
@@ -525,7 +529,7 @@ __global__ void vis_flux_les_kernel(int nu, long long E, const double* __restric
 #pragma unroll
     for (int d = 0; d < D; d++) g[k][d] = GU[i + NE * (k + (size_t)F * d)];
   }
-  vis_flux<D, double>(ph, q, g, f);
+  vis_flux_fast<D, double>(ph, q, g, f);
 #pragma unroll
   for (int k = 0; k < F; k++)
 #pragma unroll
@@ -559,7 +563,7 @@ __global__ void grad_transform_kernel(int nu, long long E, int F, double* __rest
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)nu * E) return;
   size_t NE = (size_t)nu * E;
-  double inv = 1.0 / detj[i];
+  const double inv = fr_rcp(detj[i]);
   const double* G = JG + (size_t)D * D * i;
   double Gm[D][D];
 #pragma unroll
@@ -667,8 +671,8 @@ __global__ void common_vis_kernel(int nfpi, int ni, double* const* __restrict__ 
   }
 #pragma unroll
   for (int d = 0; d < D; d++) nn[d] = *n_p[t + n * d];
-  vis_flux<D, double>(ph, ul, gl, fl);
-  vis_flux<D, double>(ph, ur, gr, fr);
+  vis_flux_fast<D, double>(ph, ul, gl, fl);
+  vis_flux_fast<D, double>(ph, ur, gr, fr);
   if (sl_p) {
 #pragma unroll
     for (int d = 0; d < D; d++)

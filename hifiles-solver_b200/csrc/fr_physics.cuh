@@ -111,77 +111,18 @@ __device__ __forceinline__ void inv_flux(const PhysT<T>& ph, const T* u, T (*f)[
 }
 
 // Viscous flux, no turbulence model: calc_visf_2d / calc_visf_3d,
-// src/flux.cpp:132-431.  With fix_vis == 1 the viscosity is mu_inf (the value
-// mu + fix_vis*(mu_inf - mu) takes whenever the Sutherland value is within a
-// factor 2 of mu_inf); otherwise Sutherland's law.
-template <int D, typename T>
-__device__ __forceinline__ void vis_flux(const PhysT<T>& ph, const T* u, T (*g)[D], T (*f)[D])
-{
-  constexpr int F = D + 2;
-  const T rho = u[0];
-  T v[D];
-#pragma unroll
-  for (int l = 0; l < D; l++) v[l] = u[l + 1] / rho;
-  T ke = v[0] * v[0];
-#pragma unroll
-  for (int l = 1; l < D; l++) ke = ke + v[l] * v[l];
-  T inte = u[F - 1] / rho - T(0.5) * ke;
-  T mu;
-  if (ph.fix_vis == T(1)) {
-    mu = ph.mu_inf;
-  } else {
-    T rt = ph.gm1 * inte / ph.rt_inf;
-    mu = ph.mu_inf * fr_pow15<T>(rt) * (T(1) + ph.c_sth) / (rt + ph.c_sth);
-    mu = mu + ph.fix_vis * (ph.mu_inf - mu);
-  }
-  T dv[D][D];   // dv[m][l] = d v_m / d x_l
-#pragma unroll
-  for (int m = 0; m < D; m++)
-#pragma unroll
-    for (int l = 0; l < D; l++) dv[m][l] = (g[m + 1][l] - g[0][l] * v[m]) / rho;
-  T de[D];
-#pragma unroll
-  for (int l = 0; l < D; l++) {
-    T vdv = v[0] * dv[0][l];
-#pragma unroll
-    for (int m = 1; m < D; m++) vdv = vdv + v[m] * dv[m][l];
-    T dke = T(0.5) * ke * g[0][l] + rho * vdv;
-    de[l] = (g[F - 1][l] - dke - g[0][l] * inte) / rho;
-  }
-  T dsum = dv[0][0];
-#pragma unroll
-  for (int l = 1; l < D; l++) dsum = dsum + dv[l][l];
-  const T diag = dsum / T(3.0);
-  const T kt = mu / ph.prandtl;   // (mu/prandtl + mu_t/prandtl_t) with mu_t = 0
-  T tau[D][D];
-#pragma unroll
-  for (int m = 0; m < D; m++)
-#pragma unroll
-    for (int l = 0; l < D; l++)
-      tau[m][l] = (m == l) ? T(2.0) * mu * (dv[m][m] - diag) : mu * (dv[m][l] + dv[l][m]);
-#pragma unroll
-  for (int l = 0; l < D; l++) {
-    f[0][l] = T(0);
-    T w = v[0] * tau[0][l];
-#pragma unroll
-    for (int m = 0; m < D; m++) {
-      f[m + 1][l] = -tau[m][l];
-      if (m > 0) w = w + v[m] * tau[m][l];
-    }
-    f[F - 1][l] = -(w + kt * ph.gamma * de[l]);
-  }
-}
-
-// The same viscous flux with one reciprocal of rho and explicit FMAs.  Used
-// where the result only enters through the viscous terms, whose size is
-// ~1/Re of the inviscid flux they are added to: its ulp-level differences from
-// the reference's division form stay far below the rounding of the total flux.
-
-// Shared part of the viscous flux, calc_visf_3d (src/flux.cpp:263-431), taken
-// one column of the gradient at a time so that a caller never holds more than
-// one: vis_begin from the state, vis_column for every direction l with g[k] =
-// d u_k / d x_l, then vis_end for the stress tau and the heat-flux term
-// q[l] = (mu gamma / Pr) de/dx_l.
+// src/flux.cpp:132-431, with one reciprocal of rho and explicit FMAs in place
+// of the reference's two dozen divisions: the result only enters through the
+// viscous terms, whose size is ~1/Re of the inviscid flux they are added to, so
+// its ulp-level differences stay far below the rounding of the total flux.
+// With fix_vis == 1 the viscosity is mu_inf (the value mu + fix_vis*(mu_inf -
+// mu) takes whenever the Sutherland value is within a factor 2 of mu_inf);
+// otherwise Sutherland's law.
+//
+// The shared part is taken one column of the gradient at a time so that a
+// caller never holds more than one: vis_begin from the state, vis_column for
+// every direction l with g[k] = d u_k / d x_l, then vis_end for the stress tau
+// and the heat-flux term q[l] = (mu gamma / Pr) de/dx_l.
 template <int D, typename T>
 struct VisState {
   T v[D], rho, ri, ke, inte, mu, kg;
