@@ -6,8 +6,7 @@
 // interpolated to each cubature point with the dense nodal-basis rows
 // opp_volume_cubpts (column order, as the reference's loop), the quantities
 // are formed with the reference's expressions, and weight x detJ at the
-// cubature point integrates them.  One thread per (element, cubature point);
-// per-block partial sums, added by fr_diag_finalize in a fixed order, so the
+// cubature point integrates them.  Per-block partial sums, added by fr_diag_finalize in a fixed order, so the
 // result does not depend on scheduling.
 #include <cuda_runtime.h>
 
@@ -15,88 +14,124 @@ namespace frb {
 
 constexpr int kDiagQ = 5;
 
-// Shared-memory order of an element's data: per solution point its C values
-// (state, then with NQ 5 the gradient), padded to an even stride so that a
-// thread reads two per load.
+// Values per point: the state, then with NQ 5 the gradient.
 template <int D, int NQ>
 struct DiagPlan {
-  static constexpr int F = D + 2, C = NQ > 1 ? F * (D + 1) : F, LD = (C + 1) / 2 * 2 + (NQ > 1 ? 2 : 0);
+  static constexpr int F = D + 2, C = NQ > 1 ? F * (D + 1) : F;
 };
-constexpr int kDiagThreads = 128;
-constexpr size_t kDiagSmemCap = 90 * 1024;   // two or more blocks per SM
+constexpr int kDiagThreads = 128, kDiagWarps = kDiagThreads / 32;
+constexpr int kDiagRows = 32, kDiagLdv = kDiagRows + 4;   // cubature points per pass, and their stride
+constexpr int kDiagTN = 5;                                // 8-column tiles per warp unit
 
-// elements per block: one thread per cubature point as far as shared memory allows
-template <int D, int NQ>
-int diag_epb(int nu, int nc)
+// smallest leading dimension >= ceil4(nu) that is 4 or 12 mod 16
+__host__ __device__ inline int diag_ld(int nu)
 {
-  const size_t per = sizeof(double) * (size_t)nu * DiagPlan<D, NQ>::LD;
-  const int by_points = nc < kDiagThreads ? kDiagThreads / nc : 1;
-  const int by_smem = (int)(kDiagSmemCap / per);
-  const int e = by_points < by_smem ? by_points : by_smem;
-  return e < 1 ? 1 : e;
+  int x = (nu + 3) / 4 * 4;
+  while (x % 16 != 4 && x % 16 != 12) x++;
+  return x;
+}
+inline size_t diag_smem(int nu, int cols) { return sizeof(double) * (size_t)((cols + 7) / 8 * 8) * (diag_ld(nu) + kDiagLdv); }
+
+// elements per block: columns for whole units of tiles, within 100 KB
+template <int D, int NQ>
+int diag_epb(int nu)
+{
+  int e = NQ > 1 && D == 3 ? 4 : 8;
+  while (e > 1 && diag_smem(nu, e * DiagPlan<D, NQ>::C) > 100 * 1024) e /= 2;
+  return e;
 }
 
 // NQ 5: all five quantities (G, the corrected gradient (nu, E, F, D), is
 // read); NQ 1: the kinetic energy alone (G unused).  Bound: the interpolation,
 // nu x C multiply-adds per cubature point (hex P = 3: 34.6 k per element, FP64
-// pipe).  A block stages its elements' state and gradient in shared memory
-// once (coalesced), and a thread carries all C values of its cubature point
-// through one pass over the solution points: per point one operator entry
-// from the L1 cache and C / 2 16-byte shared loads (broadcasts within an
-// element) feed C FMAs.  Reading state and gradient per cubature point from
-// global memory took 430 us (five quantities, 24^3 hexes of P = 3) where this
-// takes 44.
+// rate).  It is a product of the operator rows with the block's columns
+// (element, value), on the FP64 tensor cores (m8n8k4, the columns as they lie
+// in global memory): one 8-byte shared load feeds 256 multiply-adds, where a
+// thread per cubature point spends a broadcast 16-byte load per two, and was
+// bound by those (five quantities of 24^3 hexes of P = 3: 141 us; reading
+// state and gradient from global memory per point, 430).  32 cubature points a
+// pass; a thread then forms the quantities of one point.
 template <int D, typename TG, int NQ>
 __global__ void __launch_bounds__(kDiagThreads)
 fr_diag_kernel(const double* __restrict__ U, const TG* __restrict__ G, const double* __restrict__ opp,
                const double* __restrict__ W, const double* __restrict__ detj, long long E, int nu, int nc,
-               double gamma, int epb, double* __restrict__ partial)
+               double gamma, int epb, int ldk, double* __restrict__ partial)
 {
-  using Q = DiagPlan<D, NQ>;
-  constexpr int F = D + 2, C = Q::C, LD = Q::LD;
-  extern __shared__ __align__(16) double diag_smem[];
-  __shared__ double red[NQ][kDiagThreads / 32];
+  constexpr int F = D + 2, C = DiagPlan<D, NQ>::C;
+  extern __shared__ __align__(16) double diag_smem_buf[];
+  __shared__ double red[NQ][kDiagWarps];
+  const int ncol = epb * C, NTL = (ncol + 7) / 8, KS = (nu + 3) / 4;
+  double* sB = diag_smem_buf;               // [column][ldk]
+  double* sV = sB + (size_t)NTL * 8 * ldk;  // [column][kDiagLdv]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
   double acc[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; q++) acc[q] = 0.0;
+  // padding rows and columns hold zeros, or an earlier element's values
+  for (int i = tid; i < NTL * 8 * ldk; i += kDiagThreads) sB[i] = 0.0;
   for (long long e0 = (long long)blockIdx.x * epb; e0 < E; e0 += (long long)gridDim.x * epb) {
     const int nval = (int)(E - e0 < epb ? E - e0 : epb), run = nval * nu;
     __syncthreads();   // the elements before have been read
-    for (int r = threadIdx.x; r < run; r += kDiagThreads) {
-      double* dst = diag_smem + (size_t)r * LD;
+    for (int r = tid; r < run; r += kDiagThreads) {
+      const int el = r / nu;
+      double* dst = sB + (size_t)el * C * ldk + (r - el * nu);
       const size_t src = (size_t)nu * e0 + r, st = (size_t)nu * E;
 #pragma unroll
-      for (int m = 0; m < F; m++) dst[m] = U[src + st * m];
+      for (int m = 0; m < F; m++) dst[m * ldk] = U[src + st * m];
       if constexpr (NQ > 1) {
 #pragma unroll
-        for (int m = 0; m < F * D; m++) dst[F + m] = (double)G[src + st * m];
+        for (int m = 0; m < F * D; m++) dst[(F + m) * ldk] = (double)G[src + st * m];
       }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nval * nc; i += kDiagThreads) {
-    const int el = i / nc, j = i - el * nc;
-    const long long e = e0 + el;
-    double v[(C + 1) / 2 * 2];
+    for (int j0 = 0; j0 < nc; j0 += kDiagRows) {
+    const int rows = nc - j0 < kDiagRows ? nc - j0 : kDiagRows;
+    const int MT = (rows + 7) / 8, NB = (NTL + kDiagTN - 1) / kDiagTN;
+    for (int u = warp; u < MT * NB; u += kDiagWarps) {
+      const int mt = u / NB, nt0 = (u - mt * NB) * kDiagTN, r = j0 + mt * 8 + g8;
+      double c[kDiagTN][2];
+      const double* bp[kDiagTN];
 #pragma unroll
-    for (int m = 0; m < (C + 1) / 2 * 2; m++) v[m] = 0.0;
-    const double* row = diag_smem + (size_t)el * nu * LD;
-#pragma unroll 2
-    for (int k = 0; k < nu; k++) {
-      const double o = __ldg(opp + j + (size_t)nc * k);
-#pragma unroll
-      for (int m = 0; m < C; m += 2) {
-        const double2 x = *reinterpret_cast<const double2*>(row + k * LD + m);
-        v[m] = fma(o, x.x, v[m]);
-        if (m + 1 < C) v[m + 1] = fma(o, x.y, v[m + 1]);
+      for (int j = 0; j < kDiagTN; j++) {
+        c[j][0] = c[j][1] = 0.0;
+        bp[j] = sB + (size_t)((nt0 + j < NTL ? nt0 + j : nt0) * 8 + g8) * ldk + t4;
       }
+      for (int k0 = 0; k0 < KS; k0 += 8) {
+        double a[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int k = (k0 + i) * 4 + t4;
+          a[i] = (r < nc && k < nu) ? __ldg(opp + r + (size_t)nc * k) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          if (k0 + i < KS)
+#pragma unroll
+            for (int j = 0; j < kDiagTN; j++)
+              asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                  : "+d"(c[j][0]), "+d"(c[j][1])
+                  : "d"(a[i]), "d"(bp[j][(k0 + i) * 4]));
+      }
+#pragma unroll
+      for (int j = 0; j < kDiagTN; j++)
+        if (nt0 + j < NTL) {
+          double* v = sV + (size_t)((nt0 + j) * 8 + 2 * t4) * kDiagLdv + mt * 8 + g8;
+          v[0] = c[j][0];
+          v[kDiagLdv] = c[j][1];
+        }
     }
+    __syncthreads();
+    for (int i = tid; i < nval * rows; i += kDiagThreads) {
+    const int el = i / rows, jj = i - el * rows, j = j0 + jj;
+    const long long e = e0 + el;
+    const double* v = sV + (size_t)el * C * kDiagLdv + jj;
     double u[F], g[F][D];
 #pragma unroll
     for (int m = 0; m < F; m++) {
-      u[m] = v[m];
+      u[m] = v[m * kDiagLdv];
       if constexpr (NQ > 1) {
 #pragma unroll
-        for (int n = 0; n < D; n++) g[m][n] = v[F + m + F * n];
+        for (int n = 0; n < D; n++) g[m][n] = v[(F + m + F * n) * kDiagLdv];
       }
     }
     const double wj = W[j], dj = detj[j + (size_t)nc * e];
@@ -161,19 +196,20 @@ fr_diag_kernel(const double* __restrict__ U, const TG* __restrict__ G, const dou
       acc[4 % NQ] += dsc * wj * dj;
     }
     }
+    __syncthreads();   // the values have been read
+    }
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
     double v = acc[q];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) red[q][wid] = v;
+    if (lane == 0) red[q][warp] = v;
   }
   __syncthreads();
   if (threadIdx.x < NQ) {
     double v = 0.0;
-    for (int w = 0; w < kDiagThreads / 32; w++) v += red[threadIdx.x][w];
+    for (int w = 0; w < kDiagWarps; w++) v += red[threadIdx.x][w];
     partial[(size_t)blockIdx.x * NQ + threadIdx.x] = v;
   }
 }
@@ -198,14 +234,15 @@ cudaError_t diag_launch(const double* U, const TG* G, const double* opp, const d
                         long long E, int nu, int nc, double gamma, double* partial, int nblk, double* out,
                         cudaStream_t st)
 {
-  const int epb = diag_epb<D, NQ>(nu, nc);
-  const size_t sm = sizeof(double) * (size_t)epb * nu * DiagPlan<D, NQ>::LD;
+  const int epb = diag_epb<D, NQ>(nu);
+  const size_t sm = diag_smem(nu, epb * DiagPlan<D, NQ>::C);
   if (cudaError_t e = cudaFuncSetAttribute(fr_diag_kernel<D, TG, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)sm))
     return e;
   const long long groups = (E + epb - 1) / epb;
   const int grid = (int)(groups < nblk ? groups : nblk);
-  fr_diag_kernel<D, TG, NQ><<<grid, kDiagThreads, sm, st>>>(U, G, opp, W, detj, E, nu, nc, gamma, epb, partial);
+  fr_diag_kernel<D, TG, NQ><<<grid, kDiagThreads, sm, st>>>(U, G, opp, W, detj, E, nu, nc, gamma, epb, diag_ld(nu),
+                                                          partial);
   fr_diag_finalize<<<1, 32 * NQ, 0, st>>>(partial, grid, NQ, out);
   return cudaGetLastError();
 }
