@@ -42,7 +42,7 @@ __device__ __forceinline__ void upd_slot(const MergedUpd<TC>& u, long long b)
 template <typename TC, int MINB>
 __global__ void __launch_bounds__(kMergedNT, MINB) fr_merged_grad_kernel(const __grid_constant__ MergedGrads<TC> a)
 {
-  long long b = grid_block(a.rev);
+  long long b = blockIdx.x;
   if (b < a.s[0].nblk) { grad_slot<2, TC>(a.s[0], b); return; }
   b -= a.s[0].nblk;
   if (b < a.s[1].nblk) { grad_slot<3>(a.s[1], b); return; }
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kMergedNT, MINB) fr_merged_grad_kernel(const _
 template <typename TC>
 __global__ void __launch_bounds__(128) fr_merged_face_kernel(const __grid_constant__ MergedFaces<TC> a)
 {
-  long long b = grid_block(a.rev);
+  long long b = blockIdx.x;
   for (int k = 0; k < 3; k++) {
     const MergedFace<TC>& f = a.s[k];
     if (b < f.nblk) {
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(128) fr_merged_face_kernel(const __grid_consta
 template <typename TC, int MINB>
 __global__ void __launch_bounds__(kMergedNT, MINB) fr_merged_upd_kernel(const __grid_constant__ MergedUpds<TC> a)
 {
-  long long b = grid_block(a.rev);
+  long long b = blockIdx.x;
   if (b < a.s[0].nblk) { upd_slot<2>(a.s[0], b); return; }
   b -= a.s[0].nblk;
   if (b < a.s[1].nblk) { upd_slot<3>(a.s[1], b); return; }

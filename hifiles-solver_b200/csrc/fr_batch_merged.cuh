@@ -53,11 +53,10 @@ struct MergedUpd {
   int first_stage;
 };
 
-// Slot k of each launch holds the group of order k + 2 (nblk 0: no such group);
-// rev: the direction of the launch (grid_block).
-template <typename TC> struct MergedGrads { MergedGrad<TC> s[3]; int rev; };
-template <typename TC> struct MergedFaces { MergedFace<TC> s[3]; int rev; };
-template <typename TC> struct MergedUpds { MergedUpd<TC> s[3]; int rev; };
+// Slot k of each launch holds the group of order k + 2 (nblk 0: no such group).
+template <typename TC> struct MergedGrads { MergedGrad<TC> s[3]; };
+template <typename TC> struct MergedFaces { MergedFace<TC> s[3]; };
+template <typename TC> struct MergedUpds { MergedUpd<TC> s[3]; };
 
 // Host: launch the three merged kernels of one stage (faces only when some
 // group needs the separate interface kernel).  minb: CTAs per SM the

@@ -33,14 +33,6 @@ namespace frb {
 
 constexpr int kMaxN1 = 6;   // P <= 5 in the fused kernels
 
-// Order in which a grid walks over its element blocks: forwards, or with rev
-// backwards.  The kernels of a stage take turns, so that each starts with the
-// elements that the one before it has just left in the L2 cache.
-__device__ __forceinline__ long long grid_block(int rev)
-{
-  return rev ? (long long)gridDim.x - 1 - blockIdx.x : (long long)blockIdx.x;
-}
-
 template <typename T>
 struct Line {               // 1-D operator pieces (see Line1D in fr_host.hpp)
   T Lm[kMaxN1], Lp[kMaxN1], D[kMaxN1][kMaxN1], gL[kMaxN1], gR[kMaxN1], w[kMaxN1];
@@ -60,7 +52,7 @@ struct Shape {
 // axis, and whether the face is at the +1 end.  Reference orderings:
 // quads src/eles_quads.cpp:259-300, hexes src/eles_hexas.cpp:262-324.
 template <int DIM, int P>
-__host__ __device__ constexpr void fpt_line(int f, int& u0, int& stride, int& axis, bool& plus)
+__device__ __forceinline__ void fpt_line(int f, int& u0, int& stride, int& axis, bool& plus)
 {
   constexpr int N1 = P + 1;
   if (DIM == 2) {
@@ -139,7 +131,7 @@ __device__ __forceinline__ T line_interp(const Line<T>& L, const S* s, int sst, 
 }
 
 template <int DIM, int P>
-__host__ __device__ constexpr void upt_abc(int u, int& a, int& b, int& c)
+__device__ __forceinline__ void upt_abc(int u, int& a, int& b, int& c)
 {
   constexpr int N1 = P + 1;
   if (DIM == 2) { b = u / N1; a = u - b * N1; c = 0; }
@@ -151,41 +143,6 @@ __device__ __forceinline__ int upt_stride(int axis)
 {
   constexpr int N1 = P + 1;
   return axis == 0 ? 1 : (axis == 1 ? N1 : N1 * N1);
-}
-
-// The line through every flux point, packed at compile time: first point
-// (a, b, c), 3 bits each, axis << 9, plus end << 11.  A thread with a flux point
-// of its own reads its entry instead of working it out (a divergent switch over
-// the faces and three divisions).
-template <int DIM, int P>
-struct FptTable {
-  unsigned short v[Shape<DIM, P>::NF];
-  constexpr FptTable() : v()
-  {
-    for (int f = 0; f < Shape<DIM, P>::NF; f++) {
-      int u0 = 0, st = 0, ax = 0, a = 0, b = 0, c = 0;
-      bool plus = false;
-      fpt_line<DIM, P>(f, u0, st, ax, plus);
-      upt_abc<DIM, P>(u0, a, b, c);
-      v[f] = (unsigned short)(a | (b << 3) | (c << 6) | (ax << 9) | ((plus ? 1 : 0) << 11));
-    }
-  }
-};
-template <int DIM, int P>
-__device__ const FptTable<DIM, P> fpt_table = FptTable<DIM, P>();
-
-struct FptLine {
-  int a, b, c, ax;
-  bool plus;
-};
-template <int DIM, int P>
-__device__ __forceinline__ unsigned fpt_code(int f)
-{
-  return __ldg(&fpt_table<DIM, P>.v[f]);
-}
-__device__ __forceinline__ FptLine fpt_unpack(unsigned q)
-{
-  return FptLine{(int)(q & 7), (int)(q >> 3 & 7), (int)(q >> 6 & 7), (int)(q >> 9 & 3), (q >> 11 & 1) != 0};
 }
 
 // Faces at the two ends of the lines along axis d (minus end, plus end).
@@ -438,9 +395,7 @@ __host__ __device__ constexpr size_t grad_smem_bytes()
 // issue, 60 k FP64 instructions per hex P = 3 element (948 cycles of an SM).
 // One output per thread instead, each reading its line and its operator row
 // from shared memory behind run-time index arithmetic, took 5.5 k warp
-// instructions per element of which a third were FP64.  A stage's gradient
-// kernel, us: 32^3 P = 3 FP64 325 -> 285, FP32 258 -> 213; 4845 hexes P = 4 169
-// -> 93; 18000 hexes P = 2 with WALE 225 -> 191; 13031 quads P = 4 57 -> 42.
+// instructions per element of which a third were FP64.
 // The neighbours' traces go to registers (two dependent loads, issued before
 // the wait for the staged state); state, JGinv and detJ reach shared memory
 // through cp.async.  VEC = 0 keeps every global read element-sized (inputs
@@ -690,9 +645,7 @@ fr_grad_body(long long blk0, long long bstride, const double* __restrict__ U, co
   const int qe = tid / NF, qf = tid - qe * NF;
   const bool qlive = tid < EPB * NF && qe < nval;
   TC nrm[D];
-  unsigned fcode = 0;
   if constexpr (IF == 1) {
-    fcode = fpt_code<DIM, P>(qlive ? qf : 0);
     if (qlive) {
 #pragma unroll
       for (int d = 0; d < D; d++) nrm[d] = (nL + NF * e0 + NFE * d)[(unsigned)tid];
@@ -754,9 +707,11 @@ fr_grad_body(long long blk0, long long bstride, const double* __restrict__ U, co
     const int w = tid + it * NT, pe = it ? w / NF : qe, f = it ? w - pe * NF : qf;
     if (w >= EPB * NF || pe >= nval) continue;
     const long long own = f + NF * (e0 + pe);
-    const FptLine ln = fpt_unpack(IF == 1 ? fcode : fpt_code<DIM, P>(f));
-    const bool plus = ln.plus;
-    const int base = M::slot(ln.a, ln.b, ln.c) + pe * M::N, st = ln.ax == 0 ? 1 : (ln.ax == 1 ? M::S1 : M::S2);
+    int u0, ust, ax, a, b, c;
+    bool plus;
+    fpt_line<DIM, P>(f, u0, ust, ax, plus);
+    upt_abc<DIM, P>(u0, a, b, c);
+    const int base = M::slot(a, b, c) + pe * M::N, st = ax == 0 ? 1 : (ax == 1 ? M::S1 : M::S2);
     TC uf[F], n[D], Lc[N1];
 #pragma unroll
     for (int m = 0; m <= P; m++) Lc[m] = plus ? L.Lp[m] : L.Lm[m];
@@ -830,9 +785,9 @@ __global__ void __launch_bounds__(NT, MINB)
 fr_grad_kernel(const double* __restrict__ U, const TC* __restrict__ UF, const int* __restrict__ mate,
                const unsigned char* __restrict__ side, const TC* __restrict__ JG, const TC* __restrict__ detj,
                const TC* __restrict__ nL, TC* __restrict__ VF, TC* __restrict__ ND, TC* __restrict__ DV,
-               long long E, Line<TC> L, PhysT<TC> ph, TC* __restrict__ GRAD, TC* __restrict__ BV, int rev)
+               long long E, Line<TC> L, PhysT<TC> ph, TC* __restrict__ GRAD, TC* __restrict__ BV)
 {
-  fr_grad_body<DIM, P, EPB, NT, TC, LES, VEC, PERS>(PERS ? blockIdx.x : grid_block(rev), gridDim.x, U, UF, mate, side, JG, detj, nL, VF, ND,
+  fr_grad_body<DIM, P, EPB, NT, TC, LES, VEC, PERS>(blockIdx.x, gridDim.x, U, UF, mate, side, JG, detj, nL, VF, ND,
                                                      DV, E, L, ph, GRAD, BV);
 }
 
@@ -980,9 +935,9 @@ fr_face_kernel(const int2* __restrict__ face, const unsigned char* __restrict__ 
                const TC* __restrict__ UF, const TC* __restrict__ VF, const TC* __restrict__ nL,
                const TC* __restrict__ tdA, TC* __restrict__ CF, long long NFE, PhysT<TC> ph,
                long long nbdy = 0, const int* __restrict__ bf = nullptr, const unsigned char* __restrict__ bt = nullptr,
-               const TC* __restrict__ BV = nullptr, int rev = 0)
+               const TC* __restrict__ BV = nullptr)
 {
-  fr_face_body<DIM, VISC, TC, RIEMANN>(grid_block(rev), face, fsign, nint, UF, VF, nL, tdA, CF, NFE, ph, nbdy, bf, bt, BV);
+  fr_face_body<DIM, VISC, TC, RIEMANN>(blockIdx.x, face, fsign, nint, UF, VF, nL, tdA, CF, NFE, ph, nbdy, bf, bt, BV);
 }
 
 // Block partial sums -> norms: one CTA of 256 threads per field; thread t

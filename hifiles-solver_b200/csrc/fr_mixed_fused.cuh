@@ -537,8 +537,7 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_inv_kernel(MixedType t, Mixed
 // mate has arrived; what the product's epilogue needs (divergence, register,
 // state, detJ) is copied to shared memory meanwhile.  Staging all of it in
 // shared memory took two rounds of copies with a barrier each and twice the
-// shared memory per element.  The grid runs backwards (grid_block), from the
-// elements that kernel A has just left in the L2 cache.
+// shared memory per element.
 template <int D, int VISC>
 struct FptRegs {
   static constexpr int F = D + 2;
@@ -563,7 +562,7 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, Mi
   double* sUO = msm + Q::oUO;
   double* sDJ = msm + Q::oDJb;
   const int tid = threadIdx.x, warp = tid >> 5;
-  const long long E = t.E, NT = m.NT, blk = grid_block(1), e0 = blk * EPB;
+  const long long E = t.E, NT = m.NT, e0 = (long long)blockIdx.x * EPB;
   const int nval = (int)(E - e0 < EPB ? E - e0 : EPB), nuv = nval * NU, nfv = nval * NF;
   const long long gb = t.off + (long long)NF * e0;
   const size_t NFE = (size_t)NF * E, NUE = (size_t)NU * E;
@@ -705,7 +704,7 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, Mi
         for (int i = tid & 31; i < nuv; i += 32) bs += sRes[k * EU + i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) bs += __shfl_down_sync(0xffffffffu, bs, o);
-        if ((tid & 31) == 0) t.partial[(size_t)blk * F + k] = bs;
+        if ((tid & 31) == 0) t.partial[(size_t)blockIdx.x * F + k] = bs;
       }
     }
     auto bu = [&](int n) { return sUn + n * Q::ldU; };

@@ -134,7 +134,7 @@ fr_status run(const fr_residual_args* a, double* scratch, cudaStream_t s)
       cudaFuncSetAttribute(fr_grad_kernel<DIM, P, EPB, NT, double, 0, 1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)sm);
     fr_grad_kernel<DIM, P, EPB, NT, double, 0, 1, 0><<<nblk, NT, sm, s>>>(a->disu_upts, UF, a->mate, a->side, a->JGinv_upts,
-                                                                  a->detjac_upts, a->norm_left, VF, ND, DV, E, L, ph, nullptr, nullptr, 0);
+                                                                  a->detjac_upts, a->norm_left, VF, ND, DV, E, L, ph, nullptr, nullptr);
   }
   if (a->n_int > 0) {
     unsigned g = (unsigned)((a->n_int + 127) / 128);
@@ -153,7 +153,7 @@ fr_status run(const fr_residual_args* a, double* scratch, cudaStream_t s)
     if (sm > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k<<<nblk, NT, sm, s>>>(const_cast<double*>(a->disu_upts), nullptr, nullptr, nullptr, CF, a->mate, a->side, nullptr,
                            ND, DV, a->JGinv_upts, nullptr, nullptr, nullptr, nullptr, a->div_tconf_upts, nullptr, E, L,
-                           ph, 0.0, 0.0, 0.0, 0, 1);
+                           ph, 0.0, 0.0, 0.0, 0);
   };
   if (visc) update(std::integral_constant<int, 1>());
   else update(std::integral_constant<int, 0>());

@@ -71,43 +71,35 @@ struct Runner {
   }
 };
 
-// Compiled tile variants (elements per CTA, threads per CTA, CTAs per SM) of
-// the gradient and update kernels per (dims, order); the autotuner may pick any.
-// The first entry is the default of large meshes, the one with the fewest
-// elements per CTA that of small ones.  A gradient tile has a thread for each of
-// its line tasks and solution points (and, but for the 128 threads of hex P = 4,
-// flux points), an update tile one for each of its flux points, in as few idle
-// lanes as whole warps allow.  Only variants that some mesh or precision prefers
-// are kept (hexes P = 3: FP64 gradient 285 us at 6 CTAs per SM against 298 at 8,
-// FP32 213 at 8 against 239 at 6, 32^3): a variant that ties with another is
-// picked by noise, and its first launch loads it.
+// Compiled tile variants (elements per CTA, threads per CTA) of the gradient
+// and update kernels per (dims, order); the autotuner may pick any.  The first
+// entry is the default of large meshes, the last one (fewest elements per CTA)
+// that of small ones.  A gradient tile has a thread for each of its F EPB
+// NU / (P+1) line tasks, an update tile one for each of its flux points, in as
+// few idle lanes as whole warps allow.
 template <int DIM, int P> struct Tiles;
 #define FR_TILES(D_, P_, G, U) \
   template <> struct Tiles<D_, P_> { static constexpr Tile grad[] = G; static constexpr Tile upd[] = U; };
 #define T_(...) {__VA_ARGS__}
 FR_TILES(2, 1, T_({16, 128, 5}, {4, 32}), T_({16, 128, 4}, {4, 32}))
 FR_TILES(2, 2, T_({10, 128, 5}, {2, 32}), T_({10, 128, 4}, {2, 32}))
-FR_TILES(2, 3, T_({8, 128, 5}, {2, 32}), T_({8, 128, 4}, {2, 32}))
-FR_TILES(2, 4, T_({6, 160, 4}, {1, 32}), T_({5, 128, 5}, {1, 32}))
-FR_TILES(2, 5, T_({3, 128, 5}, {1, 64}), T_({3, 128, 5}, {1, 64}))
-FR_TILES(3, 1, T_({8, 192, 4}, {1, 32}), T_({8, 192, 3}, {1, 32}))
-FR_TILES(3, 2, T_({2, 128, 5}, {1, 64, 10}), T_({4, 224, 3}, {1, 64, 8}))
-FR_TILES(3, 3, T_({1, 96, 6}, {1, 96, 8}, {1, 96, 5}, {2, 192, 3, 1}), T_({1, 96, 6}, {2, 192, 3}))
-FR_TILES(3, 4, T_({1, 128, 4}, {1, 160, 3}), T_({1, 160, 5}))
+FR_TILES(2, 3, T_({8, 128, 5}, {16, 256, 3}, {2, 32}), T_({8, 128, 4}, {16, 256, 2}, {2, 32}))
+FR_TILES(2, 4, T_({6, 160, 4}, {3, 96, 6}, {1, 32}), T_({5, 128, 5}, {10, 256, 2}, {1, 32}))
+FR_TILES(2, 5, T_({3, 128, 5}, {5, 192, 3}, {1, 64}), T_({3, 128, 5}, {7, 256, 2}, {1, 64}))
+FR_TILES(3, 1, T_({8, 192, 4}, {5, 128, 5}, {1, 32}), T_({8, 192, 3}, {5, 128, 4}, {1, 32}))
+FR_TILES(3, 2, T_({4, 224, 2}, {2, 128, 5}, {1, 64, 10}), T_({4, 224, 3}, {2, 128, 4}, {1, 64, 8}))
+FR_TILES(3, 3, T_({1, 96, 6}, {1, 96, 8}, {1, 96, 5}, {2, 192, 3}, {2, 192, 3, 1}, {1, 96, 7}),
+         T_({1, 96, 6}, {1, 96, 8}, {1, 96, 5}, {2, 192, 3}))
+FR_TILES(3, 4, T_({1, 160, 3}, {1, 160, 4}, {1, 128, 4}), T_({1, 160, 5}, {1, 160, 4}))
 #undef T_
 #undef FR_TILES
 
-// The tile of a mesh before any autotuning: the first, or the one of the fewest
-// elements where the first would leave the GPU (148 SMs) with fewer than two
-// blocks per SM.
+// The tile of a mesh before any autotuning: the first, or the last where the
+// first would leave the GPU with fewer than two blocks per SM (148 SMs).
 template <int N>
 int default_tile(const Tile (&t)[N], long long E)
 {
-  if ((E + t[0].epb - 1) / t[0].epb >= 296) return 0;
-  int m = 0;
-  for (int i = 1; i < N; i++)
-    if (t[i].epb < t[m].epb) m = i;
-  return m;
+  return (E + t[0].epb - 1) / t[0].epb >= 296 ? 0 : N - 1;
 }
 
 static void set_smem(const void* k, size_t bytes)
@@ -167,13 +159,6 @@ struct RunnerT : Runner {
     }
     return m;
   }
-  // Directions of a stage's kernels (grid_block), each against the one before:
-  // where a stage has two kernels they keep theirs, one or three alternate from
-  // stage to stage with the trace buffers.
-  bool two() const { return FU == (visc != 0); }
-  int grad_rev(int cur) const { return two() ? 0 : cur; }
-  int face_rev(int cur) const { return two() ? 0 : cur ^ 1; }
-  int upd_rev(int cur) const { return two() ? 1 : cur; }
   // whether the update kernel forms the interface fluxes itself (fr_update.cuh)
   static constexpr bool FU = update_fused<DIM, P>();
   int launches_per_stage() const override { return FU ? (visc ? 2 : 1) : (visc ? 3 : 2); }
@@ -211,7 +196,7 @@ struct RunnerT : Runner {
       }
       fr_grad_kernel<DIM, P, EPB, NT, TC, LES, MINB, 1, PERS><<<(unsigned)grid, NT, sm, s>>>(
           b.U, (const TC*)b.UF[cur], b.mate, b.side, (const TC*)b.JG, (const TC*)b.detj, (const TC*)b.nL,
-          (TC*)b.VF, (TC*)b.ND, (TC*)b.DV, E, L, ph, (TC*)b.GRAD, (TC*)b.BV, grad_rev(cur));
+          (TC*)b.VF, (TC*)b.ND, (TC*)b.DV, E, L, ph, (TC*)b.GRAD, (TC*)b.BV);
     }
   }
   void grad(const Bufs& b, int cur, cudaStream_t s) override
@@ -227,7 +212,7 @@ struct RunnerT : Runner {
     fr_face_kernel<DIM, VISC, TC, RS><<<g, 128, 0, s>>>(b.face, b.fsign, b.nint, (const TC*)b.UF[cur],
                                                          VISC ? (const TC*)b.VF : nullptr, (const TC*)b.nL,
                                                          (const TC*)b.tdA, (TC*)b.CF, E * S::NF, ph, b.nbdy, b.bf,
-                                                         b.bt, VISC ? (const TC*)b.BV : nullptr, face_rev(cur));
+                                                         b.bt, VISC ? (const TC*)b.BV : nullptr);
   }
   void face(const Bufs& b, int cur, cudaStream_t s) override
   {
@@ -266,7 +251,7 @@ struct RunnerT : Runner {
         b.U, b.REG, (TC*)b.UF[cur ^ 1], (const TC*)b.UF[cur], (const TC*)b.CF, b.mate, b.side, (const TC*)b.VF,
         (const TC*)b.ND, (const TC*)b.DV, (const TC*)b.JG, (const TC*)b.nL, (const TC*)b.tdA, b.idetj,
         (const TC*)b.BV, b.DIV, want_partial ? b.partial : nullptr, E, L, ph, kRK4A[stage], kRK4B[stage], dt,
-        stage == 0 ? 1 : 0, upd_rev(cur));
+        stage == 0 ? 1 : 0);
   }
   int merged_args(const Bufs& b, int cur, int stage, double dt, void* gv, void* fv, void* uv) const override
   {

@@ -1039,12 +1039,6 @@ fr_status merged_stage_t(fr_batch* b, int k, double dt, cudaStream_t st)
     U.s[P - 2] = u;
     any_face = any_face || f.nblk > 0;
   }
-  // each launch against the one before it: three per stage, or two (then the
-  // directions stay)
-  const int c = any_face ? b->groups[0]->cur : 0;
-  G.rev = c;
-  Fc.rev = c ^ 1;
-  U.rev = any_face ? c : 1;
   fr_status r = merged_stage_launch(sizeof(TC) == 4, &G, &Fc, any_face, &U, b->merged_minb, st);
   for (fr_solver* s : b->groups) s->cur ^= 1;
   return r;

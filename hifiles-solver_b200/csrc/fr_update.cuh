@@ -24,8 +24,7 @@
 // cp.async, the state in a padded order for the line reads of the traces.  The
 // bulk-copy version of this kernel (about a hundred copies per element issued
 // by two warps, every input through shared memory, 4.2 k warp instructions per
-// element) was bound by instruction issue.  32^3, a stage: 222 us against
-// 229 in FP64, 157 against 172 in FP32.
+// element) was bound by instruction issue.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -276,8 +275,14 @@ fr_update_body(long long blk, double* __restrict__ U, double* __restrict__ REG, 
   }
 
   // the line through a flux point: first point, axis, end
-  const unsigned fcode = IF == 1 ? fpt_code<DIM, P>(tid < nval * NF ? tid % NF : 0) : 0;
-  auto fline = [&](int f) { return fpt_unpack(IF == 1 ? fcode : fpt_code<DIM, P>(f)); };
+  struct FLine { int a, b, c, ax; bool plus; };
+  auto fline = [&](int f) {
+    FLine q;
+    int u0, st;
+    fpt_line<DIM, P>(f, u0, st, q.ax, q.plus);
+    upt_abc<DIM, P>(u0, q.a, q.b, q.c);
+    return q;
+  };
   auto trace = [&](const double* s, int st, bool plus) {
     // the opp_0 row of f in column order, (((0 + t0) + t1) + ...)
     TC acc = TC(0);
@@ -294,7 +299,7 @@ fr_update_body(long long blk, double* __restrict__ U, double* __restrict__ REG, 
     if constexpr (IF > 1) load(w, in0);
     const FptIn<D, VISC, FUSED, TC>& in = in0;
     TC c[F];
-    FptLine ln;
+    FLine ln;
     if (FUSED || !VISC) ln = fline(f);
     if constexpr (FUSED != 0) {
       const double* su = sU + el * MU::N + MU::slot(ln.a, ln.b, ln.c);
@@ -442,7 +447,7 @@ fr_update_body(long long blk, double* __restrict__ U, double* __restrict__ REG, 
     for (int it = 0; it < IF; it++) {
       const int w = tid + it * NT, el = w / NF, f = w - el * NF;
       if (w >= nval * NF) continue;
-      const FptLine ln = fline(f);
+      const FLine ln = fline(f);
       const double* su = sU + el * MU::N + MU::slot(ln.a, ln.b, ln.c);
       const int st = ln.ax == 0 ? 1 : (ln.ax == 1 ? MU::S1 : MU::S2);
 #pragma unroll
@@ -460,9 +465,9 @@ fr_update_kernel(double* __restrict__ U, double* __restrict__ REG, TC* __restric
                  const TC* __restrict__ JG, const TC* __restrict__ nL, const TC* __restrict__ tdA,
                  const double* __restrict__ idetj, const TC* __restrict__ BV, double* __restrict__ DIV,
                  double* __restrict__ partial, long long E, Line<TC> L, PhysT<TC> ph, double rk_a, double rk_b,
-                 double dt, int first_stage, int rev)
+                 double dt, int first_stage)
 {
-  fr_update_body<DIM, P, EPB, NT, VISC, MODE, TC, FUSED, RIEMANN, VEC>(grid_block(rev), U, REG, UFn, UF, CF, mate, side, VF,
+  fr_update_body<DIM, P, EPB, NT, VISC, MODE, TC, FUSED, RIEMANN, VEC>(blockIdx.x, U, REG, UFn, UF, CF, mate, side, VF,
                                                                        ND, DV, JG, nL, tdA, idetj, BV, DIV, partial,
                                                                        E, L, ph, rk_a, rk_b, dt, first_stage);
 }
