@@ -677,7 +677,7 @@ def run_b200(a, rank, world, local):
                    "parallelism": "replicas" if world > 1 else "single GPU",
                    "tiles": {"grad_elements_per_cta": tiles[0], "grad_threads": tiles[1],
                              "update_elements_per_cta": tiles[2], "update_threads": tiles[3]} if tiles else None},
-        "roofline": {"bound": "hbm", "kernel": "one RK stage = fr_grad_kernel + fr_face_update_kernel",
+        "roofline": {"bound": "hbm", "kernel": "one RK stage = fr_grad_kernel + fr_update_kernel",
                      "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / pk["hbm_gbs"], "peak_source": pk_src,
                      "alg_bytes_per_element": b_elem, "traffic": traffic,

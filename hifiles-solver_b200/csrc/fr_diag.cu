@@ -48,8 +48,8 @@ int diag_epb(int nu)
 // (element, value), on the FP64 tensor cores (m8n8k4, the columns as they lie
 // in global memory): one 8-byte shared load feeds 256 multiply-adds, where a
 // thread per cubature point spends a broadcast 16-byte load per two, and was
-// bound by those (five quantities of 24^3 hexes of P = 3: 141 us; reading
-// state and gradient from global memory per point, 430).  32 cubature points a
+// bound by those (five quantities of 24^3 hexes of P = 3: 141 us, now 86; reading
+// state and gradient from global memory per point took 430).  32 cubature points a
 // pass; a thread then forms the quantities of one point.
 template <int D, typename TG, int NQ>
 __global__ void __launch_bounds__(kDiagThreads)

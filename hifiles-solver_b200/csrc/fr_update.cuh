@@ -24,7 +24,8 @@
 // cp.async, the state in a padded order for the line reads of the traces.  The
 // bulk-copy version of this kernel (about a hundred copies per element issued
 // by two warps, every input through shared memory, 4.2 k warp instructions per
-// element) was bound by instruction issue.
+// element) was bound by instruction issue.  32^3, a stage: 222 us against
+// 229 in FP64, 156 against 172 in FP32.
 #pragma once
 
 #include <cuda_runtime.h>
