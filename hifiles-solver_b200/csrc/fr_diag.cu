@@ -32,6 +32,10 @@ __host__ __device__ inline int diag_ld(int nu)
 }
 inline size_t diag_smem(int nu, int cols) { return sizeof(double) * (size_t)((cols + 7) / 8 * 8) * (diag_ld(nu) + kDiagLdv); }
 
+// largest dynamic shared memory of a block: the device's 227 KB less the
+// kernel's own norm partials
+constexpr int kDiagSmemMax = 226 * 1024;
+
 // elements per block: columns for whole units of tiles, within 100 KB
 template <int D, int NQ>
 int diag_epb(int nu)
@@ -236,8 +240,11 @@ cudaError_t diag_launch(const double* U, const TG* G, const double* opp, const d
 {
   const int epb = diag_epb<D, NQ>(nu);
   const size_t sm = diag_smem(nu, epb * DiagPlan<D, NQ>::C);
+  // the limit belongs to the kernel, not to the call: every call sets the same
+  // one, so that it is there on each device and calls of other orders from
+  // other threads never lower it
   if (cudaError_t e = cudaFuncSetAttribute(fr_diag_kernel<D, TG, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sm))
+                                           kDiagSmemMax))
     return e;
   const long long groups = (E + epb - 1) / epb;
   const int grid = (int)(groups < nblk ? groups : nblk);

@@ -5,6 +5,8 @@ values the reference itself computed on the same mesh and state
 (tests/golden/iq_*.npz), and against the numpy restatement on the solver's
 own gradient.  Tolerance 1e-12 relative to the integral of each quantity's
 absolute value (the pressure dilatation is a cancelling sum)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -104,6 +106,33 @@ def test_integral_quantities_need_the_viscous_path():
     s = H.Solver.box(2, 3, (3, 3), (-5, -5), (5, 5), viscous=False)
     with pytest.raises(H.FrError):
         s.integral_quantities()
+
+
+def test_monitoring_from_two_threads_at_different_orders():
+    """Two threads monitor solvers of orders 2 and 3 on one device: the orders
+    share a kernel but need different amounts of shared memory, and neither call
+    may be refused or changed by the other's."""
+    solvers = []
+    for P in (2, 3):
+        s = H.Solver.box(3, P, (3, 3, 3), (0, 0, 0), (2 * np.pi,) * 3, viscous=True, gamma=1.4, mu_inf=1e-3)
+        s.set_state(np.asfortranarray(O.ic_tgv(s.geometry()["pos_upts"])))
+        solvers.append((s, s.kinetic_energy(), s.integral_quantities()))
+    start, bad = threading.Barrier(2), []
+
+    def monitor(s, ke, iq):
+        start.wait()
+        for i in range(3000):
+            try:
+                if s.kinetic_energy() != ke or s.integral_quantities() != iq:
+                    bad.append((s.order, i, "changed"))
+            except H.FrError as e:
+                bad.append((s.order, i, str(e)))
+    threads = [threading.Thread(target=monitor, args=a) for a in solvers]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, (len(bad), bad[:3])
 
 
 def test_solver_vtu_matches_host_writer(tmp_path):
