@@ -10,8 +10,9 @@
 // (forward, weight gradient, input gradient) are register-tiled FP32 products
 // over shared memory, and a CTA keeps its gradient in registers over all its
 // tiles -> one partial gradient per CTA.  fr_mlp_reduce_kernel sums the
-// partials in a fixed order, so a gradient is the same bit for bit on every
-// run on one GPU model.  fr_mlp_adam_kernel applies Adam.
+// partials in a fixed order; the number of CTAs depends on the batch alone, so
+// a gradient is the same bit for bit on every run and every GPU.
+// fr_mlp_adam_kernel applies Adam.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -36,6 +37,10 @@ constexpr int kSmW2T = 0, kSmW2 = kSmW2T + kMlpH * kMlpH, kSmH1 = kSmW2 + kMlpH 
               kSmX = kSmH2 + kMlpH * kLd, kSmO = kSmX + kMlpIn * kLd, kSmDo = kSmO + kGradWarps * kTile,
               kSmEnd = kSmDo + kTile;
 constexpr size_t kGradSmem = sizeof(float) * kSmEnd;
+// Most CTAs of the loss gradient: two for each of a B200's 148 SMs (104 KB of
+// shared memory each).  A constant and not a query, since the number of partial
+// sums decides the last bits of a gradient.
+constexpr int kGradCtas = 296;
 
 fr_status mlp_fail(fr_status s, const std::string& m)
 {
@@ -413,12 +418,7 @@ fr_status fr_mlp_loss_grad(const float* w, const float* x, const float* y, const
   static bool once = (cudaFuncSetAttribute(fr_mlp_loss_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)kGradSmem), true);
   (void)once;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-    return mlp_fail(FR_ERR_CUDA, "device query failed");
-  // two CTAs per SM (104 KB of shared memory each), at most one per tile
-  const int grid = (int)(nblk < 2LL * sms ? nblk : 2LL * sms);
+  const int grid = (int)(nblk < kGradCtas ? nblk : kGradCtas);
   fr_mlp_loss_grad_kernel<<<grid, kGradThreads, kGradSmem, st>>>(w, x, y, sw, n, inv_n, scratch);
   fr_mlp_reduce_kernel<<<(kMlpTrain + 1 + 31) / 32, 32 * kRedRows, 0, st>>>(scratch, grid, inv_n, grad, loss);
   cudaError_t e = cudaGetLastError();

@@ -62,6 +62,24 @@ def test_closure_gradient_at_tile_edges(n):
     assert rel(g.cpu().numpy(), g_ref) < 1e-4
 
 
+@pytest.mark.parametrize("n", [129, 128 * 295 + 1, 128 * 296 + 1, 128 * 700])
+def test_closure_gradient_partials_depend_on_the_batch_alone(n):
+    """One partial gradient per tile of 128 samples, 296 at most whatever the
+    GPU's number of SMs: their number decides a gradient's last bits."""
+    rng = np.random.default_rng(n)
+    dev = [torch.from_numpy(a.astype(np.float32)).cuda()
+           for a in (M.init_params(3), rng.standard_normal((n, 6)), rng.uniform(0.0, 0.5, n))]
+    g = torch.empty(H.mlp_n_trained(), dtype=torch.float32, device="cuda")
+    loss = torch.empty(1, dtype=torch.float32, device="cuda")
+    ns = H.mlp_scratch_floats(n)
+    scratch = torch.full((ns,), float("nan"), dtype=torch.float32, device="cuda")
+    H.mlp_loss_grad(dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), n, g.data_ptr(), loss.data_ptr(),
+                    scratch.data_ptr(), ns)
+    torch.cuda.synchronize()
+    used = min(-(-n // 128), 296) * (H.mlp_n_trained() + 1)
+    assert bool(torch.isfinite(scratch[:used]).all()) and bool(torch.isnan(scratch[used:]).all())
+
+
 @pytest.mark.parametrize("P,viscous", [(1, False), (2, False), (3, True)])
 def test_mixed_norms_do_not_depend_on_the_launch_shape(P, viscous):
     from hifiles_b200 import mixed as X
