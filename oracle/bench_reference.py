@@ -102,7 +102,13 @@ def run(a):
     """The reference arm on the bench configuration itself (TGV n^3, P=3):
     one single-threaded reference process per host thread, as many as the
     host memory holds (about 0.7 GB per 16^3 hexes per process, measured),
-    each timing a.steps (at most 2) RK45 steps of the full mesh."""
+    each timing a.steps (at most 2) RK45 steps of the full mesh.  Without that
+    build it prints one line that says so."""
+    if not os.path.exists(HARNESS):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU build (oracle/_ref/ref_harness) is "
+                          "not here: it is built from the reference's sources by make -C oracle "
+                          "REF=<reference checkout> ref"}))
+        return
     steps = max(1, min(a.steps, 2))
     need = 0.75e9 * (a.n / 16.0) ** 3
     avail = mem_available_bytes()
