@@ -82,16 +82,31 @@ def test_closure_gradient_partials_depend_on_the_batch_alone(n):
 
 @pytest.mark.parametrize("P,viscous", [(1, False), (2, False), (3, True)])
 def test_mixed_norms_do_not_depend_on_the_launch_shape(P, viscous):
+    """6498 triangles: more block sums than the 256 threads that add them in
+    every shape, and a tail block.  At dt 1e-12 the last stage's residual is that
+    of the initial state: the state moves by 1e-12 of its residual, and the
+    residual of a small change is at most some wave speeds times the squared
+    order over the spacing (10 x 16 / 0.175, under 1e3) times that change, so
+    1e-9 of it; a lost block sum would be a thousandth."""
     from hifiles_b200 import mixed as X
     from hifiles_b200 import seam
     from test_gpu_order_tri import EULER, tri_box
-    xv, tris = tri_box(23)           # 1058 triangles: tail blocks in every shape
+    xv, tris = tri_box(57)
     mesh = X.MixedMesh(P, xv, [(X.TRI, t) for t in tris], [10.0, 10.0], [], X.ElementOpts(vcjh_scheme_tri=1))
     u0 = np.asfortranarray(O.ic_vortex(mesh.types[X.TRI]["pos_upts"]))
     types, ints, bdys = mesh.operator_inputs({X.TRI: u0})
     ph = dict(EULER, mu_inf=1e-3, tau=1.0) if viscous else EULER
+    still = seam.FusedMixedMesh(types, ints, ph, bdys, viscous=viscous)
+    still.residual()
+    div = still.S[X.TRI]["div"].cpu().numpy().reshape(u0.shape, order="F")
+    want = np.abs(div / np.asarray(types[X.TRI]["detjac_upts"])[:, :, None]).mean(axis=(0, 1))
+    assert np.all(want > 0)
     out = []
     for g, u in ((0, 0), (1, 1), (3, 2), (4, 1)) if viscous else ((1, 1),):
+        m0 = seam.FusedMixedMesh(types, ints, ph, bdys, viscous=viscous)
+        m0.set_launch(X.TRI, g, u)
+        nrm = m0.advance(1, 1e-12, norms=True)
+        assert np.all(np.abs(nrm - want) <= 1e-9 * want), (g, u, nrm, want)
         m = seam.FusedMixedMesh(types, ints, ph, bdys, viscous=viscous)
         m.set_launch(X.TRI, g, u)
         nrm = m.advance(2, 1e-3, norms=True)
