@@ -39,11 +39,13 @@ def test_integral_quantities_match_reference(case):
     assert abs(s.kinetic_energy() - a["iq"][0]) <= 1e-12 * abs(a["iq"][0])
 
 
-# the last two: more groups of 4 or 8 elements than the kernel has blocks (740),
-# and a short last group
+# the last ones: more groups of 4 or 8 elements than the kernel has blocks (740),
+# and a short last group; few groups and a rule of 729 or 81 points, spread over
+# blocks, its last pass of 32 points a short one
 @pytest.mark.parametrize("dims,P,n,jit,rule", [(3, 3, (4, 3, 3), 0.1, 3), (3, 2, (3, 3, 3), 0.0, 4),
                                                (2, 4, (4, 5), 0.1, 6), (3, 2, (19, 17, 19), 0.1, 3),
-                                               (2, 3, (79, 77), 0.1, 3)])
+                                               (2, 3, (79, 77), 0.1, 3),
+                                               (3, 2, (3, 3, 3), 0.1, 9), (2, 3, (5, 4), 0.1, 9)])
 def test_integral_quantities_match_numpy(dims, P, n, jit, rule):
     lo, hi = [0.0] * dims, [2 * np.pi] * dims
     s = H.Solver.box(dims, P, n, lo, hi, jitter=jit, seed=3, viscous=True, gamma=1.4, prandtl=0.71,
