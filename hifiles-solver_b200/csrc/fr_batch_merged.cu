@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(128) fr_merged_face_kernel(const __grid_consta
   for (int k = 0; k < 3; k++) {
     const MergedFace<TC>& f = a.s[k];
     if (b < f.nblk) {
-      fr_face_body<3, 1, TC, 0>(b, f.face, f.fsign, f.nint, f.UF, f.VF, f.nL, f.tdA, f.CF, f.NFE, f.ph, f.nbdy, f.bf,
+      fr_face_body<3, 1, TC>(b, f.face, f.fsign, f.nint, f.UF, f.VF, f.nL, f.tdA, f.CF, f.NFE, f.ph, f.nbdy, f.bf,
                                 f.bt, f.BV);
       return;
     }

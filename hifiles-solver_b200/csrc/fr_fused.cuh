@@ -102,19 +102,13 @@ __device__ __forceinline__ int face_fpt(int fc, int a, int b, int c, int& along)
   }
 }
 
-// axis and end of face fc (reference normals: quads f0 -y, f1 +x, f2 +y, f3 -x;
+// end of face fc (reference normals: quads f0 -y, f1 +x, f2 +y, f3 -x;
 // hexes f0 -z, f1 -y, f2 +x, f3 +y, f4 -x, f5 +z)
 template <int DIM>
 __device__ __forceinline__ bool face_plus(int fc)
 {
   if (DIM == 2) return fc == 1 || fc == 2;
   return fc == 2 || fc == 3 || fc == 5;
-}
-template <int DIM>
-__device__ __forceinline__ int face_axis(int fc)
-{
-  if (DIM == 2) return (fc == 1 || fc == 3) ? 0 : 1;
-  return (fc == 2 || fc == 4) ? 0 : ((fc == 1 || fc == 3) ? 1 : 2);
 }
 
 // Value at flux point f of a field stored point-major (s[u * sst]): the
@@ -136,13 +130,6 @@ __device__ __forceinline__ void upt_abc(int u, int& a, int& b, int& c)
   constexpr int N1 = P + 1;
   if (DIM == 2) { b = u / N1; a = u - b * N1; c = 0; }
   else { c = u / (N1 * N1); int r = u - c * N1 * N1; b = r / N1; a = r - b * N1; }
-}
-
-template <int DIM, int P>
-__device__ __forceinline__ int upt_stride(int axis)
-{
-  constexpr int N1 = P + 1;
-  return axis == 0 ? 1 : (axis == 1 ? N1 : N1 * N1);
 }
 
 // Faces at the two ends of the lines along axis d (minus end, plus end).
@@ -795,7 +782,7 @@ fr_grad_kernel(const double* __restrict__ U, const TC* __restrict__ UF, const in
 
 // Boundary point j of the interface kernel (flat own index bf[j], type
 // bt[j]), out of line so that the interior path keeps few registers.
-template <int DIM, int VISC, typename TC, int RIEMANN>
+template <int DIM, int VISC, typename TC>
 __device__ __noinline__ void face_boundary(PhysT<TC> ph, long long j, const TC* __restrict__ UF,
                                            const TC* __restrict__ nL, const TC* __restrict__ tdA, TC* __restrict__ CF,
                                            long long NFE, const int* __restrict__ bf,
@@ -821,8 +808,6 @@ __device__ __noinline__ void face_boundary(PhysT<TC> ph, long long j, const TC* 
       for (int l = 1; l < D; l++) s = s + fl[k][l] * n[l];
       fn[k] = s;
     }
-  } else if (RIEMANN == 2 && DIM == 2) {
-    roe<TC>(ph, ul, ug, n, fn);
   } else {
 #pragma unroll
     for (int k = 0; k < F; k++) {
@@ -848,17 +833,16 @@ __device__ __noinline__ void face_boundary(PhysT<TC> ph, long long j, const TC* 
 // projections VF, src/int_inters.cpp:359-470).  Writes norm_tconf_fpts of
 // both sides: +f_n tdA_l on the left, -f_n tdA_r on the right.
 // face[i] = (left flat index, right flat index) of interface point i;
-// fsign[i] != 0 when the LDG penalty sign is negative there.  RIEMANN is the
-// reference's riemann_solve_type: 0 Rusanov, 2 Roe (2-D).
+// fsign[i] != 0 when the LDG penalty sign is negative there.
 // Threads past nint take the boundary points: ghost state, inviscid common
 // flux of bdy_inters::evaluate_boundaryConditions_invFlux (central flux of the
-// two states, convective_flux_boundary, src/inters.cpp:368-387; Roe in 2-D
-// with RIEMANN 2; the own flux for slip_wall_dual, right_flux,
-// src/inters.cpp:299-308), plus the viscous part BV from the gradient kernel.
+// two states, convective_flux_boundary, src/inters.cpp:368-387; the own flux
+// for slip_wall_dual, right_flux, src/inters.cpp:299-308), plus the viscous part
+// BV from the gradient kernel.
 // Blocks of exactly 128 threads (one shared staging column per thread); the
 // body serves block blk (fr_face_kernel: blockIdx.x; merged batch launches:
 // their share of the grid).
-template <int DIM, int VISC, typename TC, int RIEMANN = 0>
+template <int DIM, int VISC, typename TC>
 __device__ __forceinline__ void
 fr_face_body(long long blk, const int2* __restrict__ face, const unsigned char* __restrict__ fsign, long long nint,
              const TC* __restrict__ UF, const TC* __restrict__ VF, const TC* __restrict__ nL,
@@ -868,7 +852,7 @@ fr_face_body(long long blk, const int2* __restrict__ face, const unsigned char* 
   constexpr int F = DIM + 2, D = DIM;
   long long i = blk * 128 + threadIdx.x;
   if (i >= nint) {
-    if (i - nint < nbdy) face_boundary<DIM, VISC, TC, RIEMANN>(ph, i - nint, UF, nL, tdA, CF, NFE, bf, bt, BV);
+    if (i - nint < nbdy) face_boundary<DIM, VISC, TC>(ph, i - nint, UF, nL, tdA, CF, NFE, bf, bt, BV);
     return;
   }
   // FP64: the point's inputs reach shared memory through cp.async (one
@@ -908,8 +892,7 @@ fr_face_body(long long blk, const int2* __restrict__ face, const unsigned char* 
   for (int d = 0; d < D; d++) n[d] = in(2 * F + d, nL + a + NFE * d);
   const TC tl = in(2 * F + D, tdA + a), tr = in(2 * F + D + 1, tdA + b);
   TC fn[F];
-  if constexpr (RIEMANN == 2 && DIM == 2) roe<TC>(ph, ul, ur, n, fn);
-  else rusanov<D, TC>(ph, ul, ur, n, fn);
+  rusanov<D, TC>(ph, ul, ur, n, fn);
   TC cl[F], cr[F];
 #pragma unroll
   for (int k = 0; k < F; k++) { cl[k] = fn[k] * tl; cr[k] = -fn[k] * tr; }
@@ -931,7 +914,7 @@ fr_face_body(long long blk, const int2* __restrict__ face, const unsigned char* 
   for (int k = 0; k < F; k++) { CF[a + NFE * k] = cl[k]; CF[b + NFE * k] = cr[k]; }
 }
 
-template <int DIM, int VISC, typename TC, int RIEMANN = 0>
+template <int DIM, int VISC, typename TC>
 __global__ void __launch_bounds__(128)
 fr_face_kernel(const int2* __restrict__ face, const unsigned char* __restrict__ fsign, long long nint,
                const TC* __restrict__ UF, const TC* __restrict__ VF, const TC* __restrict__ nL,
@@ -939,7 +922,7 @@ fr_face_kernel(const int2* __restrict__ face, const unsigned char* __restrict__ 
                long long nbdy = 0, const int* __restrict__ bf = nullptr, const unsigned char* __restrict__ bt = nullptr,
                const TC* __restrict__ BV = nullptr)
 {
-  fr_face_body<DIM, VISC, TC, RIEMANN>(blockIdx.x, face, fsign, nint, UF, VF, nL, tdA, CF, NFE, ph, nbdy, bf, bt, BV);
+  fr_face_body<DIM, VISC, TC>(blockIdx.x, face, fsign, nint, UF, VF, nL, tdA, CF, NFE, ph, nbdy, bf, bt, BV);
 }
 
 // Block partial sums -> norms: one CTA of 256 threads per field; thread t

@@ -47,6 +47,7 @@ struct Runner {
   virtual int flux_blocks() const = 0;      // blocks of the update kernel (norm partials)
   virtual int max_flux_blocks() const = 0;  // over all update-kernel tiles
   virtual int launches_per_stage() const = 0;
+  virtual bool forms_interface_fluxes() const = 0;   // in the update kernel: no face kernel, CF is not touched
   virtual void set_riemann(int rs) = 0;
   // tile variants of the two element kernels (autotuning)
   virtual int n_grad_tiles() const = 0;
@@ -81,7 +82,6 @@ struct RunnerT : Runner {
   int visc, les, riemann = 0;
   int gsel = 0, usel = 0;
   Line<TC> L;
-  Line<double> L64;
   PhysT<TC> ph;
   RunnerT(long long E_, int visc_, int les_, const Line1D& l, const Phys& p) : E(E_), visc(visc_), les(les_)
   {
@@ -93,11 +93,6 @@ struct RunnerT : Runner {
       L.Lm[i] = (TC)l.Lm[i]; L.Lp[i] = (TC)l.Lp[i]; L.gL[i] = (TC)l.gL[i]; L.gR[i] = (TC)l.gR[i];
       L.w[i] = (TC)l.w[i];
       for (int j = 0; j <= P; j++) L.D[i][j] = (TC)l.D[i][j];
-    }
-    for (int i = 0; i < kMaxN1; i++) {
-      L64.Lm[i] = i <= P ? l.Lm[i] : 0; L64.Lp[i] = i <= P ? l.Lp[i] : 0; L64.gL[i] = i <= P ? l.gL[i] : 0;
-      L64.gR[i] = i <= P ? l.gR[i] : 0; L64.w[i] = i <= P ? l.w[i] : 0;
-      for (int j = 0; j < kMaxN1; j++) L64.D[i][j] = (i <= P && j <= P) ? l.D[i][j] : 0;
     }
     ph = PhysT<TC>::make(p);
     gsel = default_tile(Tiles<DIM, P>::grad, E);
@@ -127,6 +122,7 @@ struct RunnerT : Runner {
   // whether the update kernel forms the interface fluxes itself (fr_update.cuh)
   static constexpr bool FU = update_fused<DIM, P>();
   int launches_per_stage() const override { return FU ? (visc ? 2 : 1) : (visc ? 3 : 2); }
+  bool forms_interface_fluxes() const override { return FU; }
   void set_riemann(int rs) override { riemann = rs; }
   void trace(const Bufs& b, int cur, cudaStream_t s, const double* src = nullptr) override
   {
@@ -170,25 +166,24 @@ struct RunnerT : Runner {
     else grad_i<0, 0>(b, cur, s);
   }
 
-  template <int VISC, int RS>
+  template <int VISC>
   void face_t(const Bufs& b, int cur, cudaStream_t s)
   {
     unsigned g = (unsigned)((b.nint + b.nbdy + 127) / 128);
-    fr_face_kernel<DIM, VISC, TC, RS><<<g, 128, 0, s>>>(b.face, b.fsign, b.nint, (const TC*)b.UF[cur],
-                                                         VISC ? (const TC*)b.VF : nullptr, (const TC*)b.nL,
-                                                         (const TC*)b.tdA, (TC*)b.CF, E * S::NF, ph, b.nbdy, b.bf,
-                                                         b.bt, VISC ? (const TC*)b.BV : nullptr);
+    fr_face_kernel<DIM, VISC, TC><<<g, 128, 0, s>>>(b.face, b.fsign, b.nint, (const TC*)b.UF[cur],
+                                                    VISC ? (const TC*)b.VF : nullptr, (const TC*)b.nL,
+                                                    (const TC*)b.tdA, (TC*)b.CF, E * S::NF, ph, b.nbdy, b.bf, b.bt,
+                                                    VISC ? (const TC*)b.BV : nullptr);
   }
   void face(const Bufs& b, int cur, cudaStream_t s) override
   {
-    if (FU || b.nint + b.nbdy == 0) return;
-    if (DIM == 2 && riemann == 2) {
-      if (visc) face_t<1, 2>(b, cur, s);
-      else face_t<0, 2>(b, cur, s);
-    } else {
-      if (visc) face_t<1, 0>(b, cur, s);
-      else face_t<0, 0>(b, cur, s);
+    // hexes of even order only, so Rusanov: the Roe flux is 2-D
+    if constexpr (!FU) {
+      if (b.nint + b.nbdy == 0) return;
+      if (visc) face_t<1>(b, cur, s);
+      else face_t<0>(b, cur, s);
     }
+    (void)b; (void)cur; (void)s;
   }
 
   template <int I, int VISC, int MODE>

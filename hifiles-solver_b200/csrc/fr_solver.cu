@@ -287,7 +287,9 @@ static fr_status create_with_mesh(Mesh&& mesh, const Line1D& line, const fr_sche
     if ((st = dalloc(s.get(), &p, nf * E * F * tc))) return st; s->b.ND = p;
     if ((st = dalloc(s.get(), &p, nu * E * F * tc))) return st; s->b.DV = p;
   }
-  if ((st = dalloc(s.get(), &p, nf * E * F * tc))) return st; s->b.CF = p;
+  if (!r->forms_interface_fluxes()) {
+    if ((st = dalloc(s.get(), &p, nf * E * F * tc))) return st; s->b.CF = p;
+  }
   s->b.nint = (long long)m.il.size();
   s->b.nbdy = (long long)m.bf.size();
   if (s->b.nbdy > 0) {
