@@ -95,7 +95,7 @@ struct RunnerT : Runner {
       for (int j = 0; j <= P; j++) L.D[i][j] = (TC)l.D[i][j];
     }
     ph = PhysT<TC>::make(p);
-    gsel = default_tile(Tiles<DIM, P>::grad, E);
+    gsel = default_grad_tile<DIM, P>(E, les != 0);
     usel = default_tile(Tiles<DIM, P>::upd, E);
   }
   int n_grad_tiles() const override { return NG; }

@@ -12,8 +12,9 @@ struct Tile {
 
 // Compiled tile variants (elements per CTA, threads per CTA) of the gradient
 // and update kernels per (dims, order); the autotuner may pick any.  The first
-// entry is the default of large meshes, the last of those with the fewest
-// elements per CTA that of small ones.  A gradient tile has a thread for each
+// entry is the default of large meshes (hexes of P = 2 apart, see
+// default_grad_tile), the last of those with the fewest elements per CTA that of
+// small ones.  A gradient tile has a thread for each
 // of its F EPB NU / (P+1) line tasks, an update tile one for each of its flux
 // points, in as few idle lanes as whole warps allow.
 template <int DIM, int P> struct Tiles;
@@ -44,6 +45,18 @@ constexpr int default_tile(const Tile (&t)[N], long long E)
   for (int i = 1; i < N; i++)
     if (t[i].epb <= t[m].epb) m = i;
   return m;
+}
+
+// The gradient tile likewise, but for large meshes of hexes of P = 2 without LES
+// the second one, 2 elements on 128 threads: a stage of 21840 hexes takes 199 us
+// with it against 208 with 4 elements on 224 threads, in FP32 148 against 166.
+// The LES kernel spills more at its 96 registers than at the 128 of the first
+// (6188 walled hexes, Smagorinsky: 102.8 against 101.2 us).
+template <int DIM, int P>
+constexpr int default_grad_tile(long long E, bool les)
+{
+  const int i = default_tile(Tiles<DIM, P>::grad, E);
+  return DIM == 3 && P == 2 && i == 0 && !les ? 1 : i;
 }
 
 }  // namespace frb

@@ -28,6 +28,12 @@ template <int N> void show(const char* kind, int d, int p, const frb::Tile (&t)[
 int main()
 {
 %s
+  for (int les : {0, 1})
+    for (long long e : {8LL, 1200LL, 30000LL}) {
+      const frb::Tile t = frb::Tiles<3, 2>::grad[frb::default_grad_tile<3, 2>(e, les)];
+      std::printf("p2 %%d %%lld %%d %%d\\n", les, e, t.epb, t.nt);
+      if (frb::default_grad_tile<3, 3>(e, les) != frb::default_tile(frb::Tiles<3, 3>::grad, e)) return 1;
+    }
 }
 """
 
@@ -41,6 +47,10 @@ def test_default_tiles(tmp_path):
     exe = str(tmp_path / "tiles")
     subprocess.run(["g++", "-std=c++17", "-I", CSRC, str(src), "-o", exe], check=True)
     rows = [r.split() for r in subprocess.run([exe], check=True, capture_output=True, text=True).stdout.splitlines()]
+    hexes_p2 = [tuple(int(v) for v in r[1:]) for r in rows if r[0] == "p2"]
+    assert hexes_p2 == [(0, 8, 1, 64), (0, 1200, 2, 128), (0, 30000, 2, 128),
+                        (1, 8, 1, 64), (1, 1200, 4, 224), (1, 30000, 4, 224)]
+    rows = [r for r in rows if r[0] != "p2"]
     assert len(rows) == len(SHAPES) * 2 * len(SMALL + LARGE)
     for kind, d, p, e, i, epb, least in rows:
         if int(e) in SMALL:
