@@ -75,14 +75,14 @@ fr_status mlaunched(const char* what)
 // (dims, solution points, flux points) with kernels: tets, prisms and hexes of
 // orders 2 and 3 here, triangles and quads of orders 2 and 3 in
 // fr_mixed_fused_2d.cu, orders 1 and 4 in fr_mixed_fused_p14.cu
-bool find_kernels(int D, int NU, int NF, MixedKernels* out)
+bool find_kernels(int D, int NU, int NF, long long E, int pf, MixedKernels* out)
 {
-  if (find_kernels_p14(D, NU, NF, out)) return true;
-  if (D == 2) return find_kernels_2d(NU, NF, out);
+  if (find_kernels_p14(D, NU, NF, E, pf, out)) return true;
+  if (D == 2) return find_kernels_2d(NU, NF, E, pf, out);
   if (D != 3) return false;
 #define FR_MIXED_SHAPE(nu, nf) \
   if (NU == nu && NF == nf) {  \
-    *out = mixed_kernels<3, nu, nf>(); \
+    *out = mixed_kernels_for<3, nu, nf>(E, pf); \
     return true;               \
   }
   FR_MIXED_SHAPE(10, 24)  // tet P2
@@ -206,9 +206,8 @@ __global__ void __launch_bounds__(kNormThreads) mixed_norm_finalize(NormParts np
 fr_status launch_grad(fr_mixed_stage* s, int i, int v, const double* UFc, cudaStream_t st)
 {
   const MixedType& t = s->types[i];
-  const MixedShape& g = kGradShapes[v];
-  s->kern[i].grad[s->pf][v]<<<blocks_of(t.E, s->kern[i].epb_a[v]), g.nth, s->kern[i].smem_a[s->pf][v], st>>>(t, s->fp, UFc,
-                                                                                                 s->ph);
+  s->kern[i].grad[s->pf][v]<<<blocks_of(t.E, s->kern[i].epb_a[s->pf][v]), kGradShapes[v].nth, s->kern[i].smem_a[s->pf][v],
+                              st>>>(t, s->fp, UFc, s->ph);
   return mlaunched("mixed_grad_kernel");
 }
 
@@ -220,9 +219,9 @@ fr_status launch_upd(fr_mixed_stage* s, int i, int v, int mode, int stage, doubl
                               0.153057247968152};
   MixedType t = s->types[i];
   t.partial = norms ? s->partials[i] : nullptr;
-  const MixedShape& u = kUpdShapes[v];
   auto k = mode ? s->kern[i].upd1[s->pf][v] : s->kern[i].upd0[s->pf][v];
-  k<<<blocks_of(t.E, s->kern[i].epb_b[v]), u.nth, s->kern[i].smem_b[v], st>>>(t, s->fp, UFc, UFn, s->ph, A[stage], B[stage], dt);
+  k<<<blocks_of(t.E, s->kern[i].epb_b[s->pf][v]), s->kern[i].nth_b[s->pf][v], s->kern[i].smem_b[s->pf][v], st>>>(
+      t, s->fp, UFc, UFn, s->ph, A[stage], B[stage], dt);
   return mlaunched("mixed_update_kernel");
 }
 
@@ -284,8 +283,8 @@ fr_status set_smem(const MixedKernels& k, int pf)
   std::vector<std::pair<const void*, size_t>> list;
   for (int v = 0; v < kNGrad; v++) list.push_back({(const void*)k.grad[pf][v], k.smem_a[pf][v]});
   for (int v = 0; v < kNUpd; v++) {
-    list.push_back({(const void*)k.upd0[pf][v], k.smem_b[v]});
-    list.push_back({(const void*)k.upd1[pf][v], k.smem_b[v]});
+    list.push_back({(const void*)k.upd0[pf][v], k.smem_b[pf][v]});
+    list.push_back({(const void*)k.upd1[pf][v], k.smem_b[pf][v]});
   }
   list.push_back({(const void*)k.trace, k.smem_c});
   bool any_grad = false, any_upd = false;
@@ -352,7 +351,7 @@ fr_status fr_mixed_stage_create(int n_dims, int n_types, const fr_mixed_stage_ty
       if (!ty.opp_1[d] || !ty.opp_2[d] || (viscous && (!ty.opp_4[d] || !ty.opp_5[d])))
         return bail(mfail(FR_ERR_ARG, "missing operator"));
     MixedKernels k;
-    if (!find_kernels(D, NU, NF, &k))
+    if (!find_kernels(D, NU, NF, ty.n_eles, pf, &k))
       return bail(mfail(FR_ERR_UNSUPPORTED, "fused mixed stage: no kernels for " + std::to_string(NU) +
                                                 " solution / " + std::to_string(NF) + " flux points"));
     s->kern.push_back(k);
@@ -639,7 +638,7 @@ fr_status fr_mixed_stage_advance_norms(fr_mixed_stage* s, int n_steps, double dt
   double n_upts = 0.0;
   for (int i = 0; i < s->n_types; i++) {
     np.p[i] = s->partials[i];
-    np.nb[i] = s->types[i].E > 0 ? (int)blocks_of(s->types[i].E, s->kern[i].epb_b[s->uv[i]]) : 0;
+    np.nb[i] = s->types[i].E > 0 ? (int)blocks_of(s->types[i].E, s->kern[i].epb_b[s->pf][s->uv[i]]) : 0;
     n_upts += (double)s->types[i].NU * (double)s->types[i].E;
   }
   mixed_norm_finalize<<<s->F, kNormThreads, 0, st>>>(np, s->n_types, s->F, n_upts, s->norms_dev);

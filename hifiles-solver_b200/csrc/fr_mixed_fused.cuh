@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, Mixe
                                                                const double* __restrict__ UFc, PhysT<double> ph)
 {
   using Q = MPlan<D, NU, NF, EPB, MINB>;
-  constexpr int F = D + 2, NW = NTH / 32, DD = D * D, EU = Q::EU, EF = Q::EF;
+  constexpr int F = D + 2, NW = NTH / 32, DD = D * D, EF = Q::EF;
   extern __shared__ __align__(16) double msm[];
   double* sU = msm + Q::oU;
   double* sUF = msm + Q::oUF;
@@ -661,11 +661,8 @@ __global__ void __launch_bounds__(NTH, MINB) mixed_update_kernel(MixedType t, Mi
   // div_tconf = div_tdisf + opp_3 jump, then the RK45 update
   // (RK45_update_kernel: rhs = -div / detJ)
   {
-    if (MODE == 1)  // padding rows of the new state, read (times zero) by the trace product
-      for (int i = tid; i < Q::NP * (c4(NU) - NU); i += NTH) {
-        const int n = i / (c4(NU) - NU), r = NU + i % (c4(NU) - NU);
-        sUn[n * Q::ldU + r] = 0.0;
-      }
+    // padding rows of the new state, read (times zero) by the trace product
+    if constexpr (MODE == 1) zero_pad_rows<NU, c4(NU), Q::ldU, Q::NP, NTH>(sUn);
     auto bj = [&](int n) { return sJ + n * Q::ldF; };
     auto one = [&](int r, int n, double v) {
       const int el = n / F, k = n - el * F;
@@ -763,13 +760,13 @@ constexpr MixedShape kGradShapes[] = {{8, 256, 1}, {4, 128, 3}, {4, 160, 3}, {4,
 constexpr MixedShape kUpdShapes[] = {{8, 256, 2}, {4, 160, 3}, {4, 128, 4}};
 constexpr int kNGrad = sizeof(kGradShapes) / sizeof(kGradShapes[0]);
 constexpr int kNUpd = sizeof(kUpdShapes) / sizeof(kUpdShapes[0]);
-// Elements per block of a type with NF flux points: the shape's, or as many
-// (in fours, whole column tiles) as give each flux point a thread.  Types with
-// few points would leave most of a block idle otherwise: triangles of P = 2 had
-// 36 flux points on 128 threads (update kernel of 17280: 26.5 us).
-__host__ __device__ constexpr int shape_epb(MixedShape s, int nf)
+// Elements per block of a type with NF flux points: the shape's, or filled as
+// many (in fours, whole column tiles) as give each flux point a thread.  Types
+// with few points would leave most of a block idle otherwise: triangles of
+// P = 2 had 36 flux points on 128 threads (update kernel of 17280: 26.5 us).
+__host__ __device__ constexpr int shape_epb(MixedShape s, int nf, bool fill)
 {
-  return cmax(s.epb, s.nth / nf / 4 * 4);
+  return fill ? cmax(s.epb, s.nth / nf / 4 * 4) : s.epb;
 }
 
 using GradFn = void (*)(MixedType, MixedFpts, const double*, PhysT<double>);
@@ -777,52 +774,59 @@ using UpdFn = void (*)(MixedType, MixedFpts, const double*, double*, PhysT<doubl
 using TraceFn = void (*)(MixedType, long long, double*);
 
 // Physics forms: 0 Navier-Stokes (Rusanov + LDG), 1 Euler with Rusanov,
-// 2 Euler with Roe (2-D).  The Euler forms have one launch shape (gradient
-// slot 1: the flux kernel of 4 elements x 128 threads; update 1).
+// 2 Euler with Roe (2-D).  The Euler forms have one launch shape, slot 1 of
+// either list: the flux kernel of 4 elements x 128 threads, and the update
+// kernel of 4 x 160, or of 4 x 128 where blocks are not filled.
 constexpr int kNForms = 3;
 
 struct MixedKernels {
   int D, NU, NF;
-  int epb_a[kNGrad], epb_b[kNUpd], epb_c;  // elements per block of each launch shape
+  // elements per block of each launch shape, threads per block of the update kernels
+  int epb_a[kNForms][kNGrad], epb_b[kNForms][kNUpd], epb_c, nth_b[kNForms][kNUpd];
   GradFn grad[kNForms][kNGrad];
   size_t smem_a[kNForms][kNGrad];
   UpdFn upd0[kNForms][kNUpd], upd1[kNForms][kNUpd];
-  size_t smem_b[kNUpd];
+  size_t smem_b[kNForms][kNUpd];
   TraceFn trace;
   size_t smem_c;
 };
 
-template <int D, int NU, int NF, int V>
+template <int D, int NU, int NF, bool FILL, int V>
 void fill_grad(MixedKernels& k)
 {
   constexpr MixedShape g = kGradShapes[V];
-  constexpr int epb = shape_epb(g, NF);
-  k.epb_a[V] = epb;
+  constexpr int epb = shape_epb(g, NF, FILL);
+  k.epb_a[0][V] = epb;
   k.smem_a[0][V] = sizeof(double) * MPlan<D, NU, NF, epb, g.minb>::nA;
   k.grad[0][V] = k.smem_a[0][V] <= kMixedSmemMax ? mixed_grad_kernel<D, NU, NF, epb, g.nth, g.minb> : nullptr;
 }
 
-template <int D, int NU, int NF, int V>
+template <int D, int NU, int NF, bool FILL, int V>
 void fill_upd(MixedKernels& k)
 {
   constexpr MixedShape u = kUpdShapes[V];
-  constexpr int epb = shape_epb(u, NF);
-  k.epb_b[V] = epb;
-  k.smem_b[V] = sizeof(double) * MPlan<D, NU, NF, epb>::nB;
-  const bool fits = k.smem_b[V] <= kMixedSmemMax;
+  constexpr int epb = shape_epb(u, NF, FILL);
+  k.epb_b[0][V] = epb;
+  k.nth_b[0][V] = u.nth;
+  k.smem_b[0][V] = sizeof(double) * MPlan<D, NU, NF, epb>::nB;
+  const bool fits = k.smem_b[0][V] <= kMixedSmemMax;
   k.upd0[0][V] = fits ? mixed_update_kernel<D, NU, NF, epb, u.nth, u.minb, 0> : nullptr;
   k.upd1[0][V] = fits ? mixed_update_kernel<D, NU, NF, epb, u.nth, u.minb, 1> : nullptr;
 }
 
-template <int D, int NU, int NF>
+template <int D, int NU, int NF, bool FILL>
 void fill_euler(MixedKernels& k)
 {
-  constexpr MixedShape g = kGradShapes[1], u = kUpdShapes[1];
-  constexpr int ge = shape_epb(g, NF), ue = shape_epb(u, NF);
-  const size_t sa = sizeof(double) * MPlanInv<D, NU, NF, ge>::nI;
-  const bool fa = sa <= kMixedSmemMax, fb = k.smem_b[1] <= kMixedSmemMax;
+  constexpr MixedShape g = kGradShapes[1], u = kUpdShapes[FILL ? 1 : 2];
+  constexpr int ge = shape_epb(g, NF, FILL), ue = shape_epb(u, NF, FILL);
+  const size_t sa = sizeof(double) * MPlanInv<D, NU, NF, ge>::nI, sb = sizeof(double) * MPlan<D, NU, NF, ue>::nB;
+  const bool fa = sa <= kMixedSmemMax, fb = sb <= kMixedSmemMax;
   for (int f = 1; f < kNForms; f++) {
+    k.epb_a[f][1] = ge;
+    k.epb_b[f][1] = ue;
+    k.nth_b[f][1] = u.nth;
     k.smem_a[f][1] = sa;
+    k.smem_b[f][1] = sb;
     k.grad[f][1] = fa ? mixed_inv_kernel<D, NU, NF, ge, g.nth, g.minb> : nullptr;
   }
   k.upd0[1][1] = fb ? mixed_update_kernel<D, NU, NF, ue, u.nth, u.minb, 0, 0, 0> : nullptr;
@@ -833,24 +837,27 @@ void fill_euler(MixedKernels& k)
   }
 }
 
-template <int D, int NU, int NF>
+// Without FILL, the shapes that a stage starts with (gradient 3, update 1, and
+// the Euler forms) keep their own number of elements; the others are filled
+// all the same, so that every shape is there for meshes of any size.
+template <int D, int NU, int NF, bool FILL>
 MixedKernels mixed_kernels()
 {
   MixedKernels k{};
   k.D = D;
   k.NU = NU;
   k.NF = NF;
-  fill_grad<D, NU, NF, 0>(k);
-  fill_grad<D, NU, NF, 1>(k);
-  fill_grad<D, NU, NF, 2>(k);
-  fill_grad<D, NU, NF, 3>(k);
-  fill_grad<D, NU, NF, 4>(k);
-  fill_upd<D, NU, NF, 0>(k);
-  fill_upd<D, NU, NF, 1>(k);
-  fill_upd<D, NU, NF, 2>(k);
+  fill_grad<D, NU, NF, true, 0>(k);
+  fill_grad<D, NU, NF, true, 1>(k);
+  fill_grad<D, NU, NF, true, 2>(k);
+  fill_grad<D, NU, NF, FILL, 3>(k);
+  fill_grad<D, NU, NF, true, 4>(k);
+  fill_upd<D, NU, NF, true, 0>(k);
+  fill_upd<D, NU, NF, FILL, 1>(k);
+  fill_upd<D, NU, NF, true, 2>(k);
   static_assert(kNGrad == 5 && kNUpd == 3, "one fill per shape");
-  fill_euler<D, NU, NF>(k);
-  constexpr int te = shape_epb(MixedShape{kMixedEPB, kMixedNT, 1}, NF);
+  fill_euler<D, NU, NF, FILL>(k);
+  constexpr int te = shape_epb(MixedShape{kMixedEPB, kMixedNT, 1}, NF, true);
   k.epb_c = te;
   k.trace = mixed_trace_kernel<D, NU, NF, te, kMixedNT>;
   k.smem_c = sizeof(double) * MPlan<D, NU, NF, te>::nC;
@@ -858,9 +865,28 @@ MixedKernels mixed_kernels()
 }
 
 
+// The kernels of a type of E elements, for physics form pf.  Filling the blocks
+// pays where they would otherwise come in more than one wave; a mesh whose
+// blocks of 4 elements are all resident at once is bound by the latency of one
+// block, which grows with its elements.  Blocks of 4 elements resident per SM:
+// three of the viscous update kernel, five of the Euler one, four with the Roe
+// flux; where filling only doubles the elements, a second wave of Euler blocks
+// is no slower either.  A stage, us, blocks of 4 elements / filled: triangles of
+// P = 3 Navier-Stokes, 1404: 12.6 / 14.7, 2520: 18.7 / 16.7, 8448: 34.7 / 28.9;
+// Euler 1984: 10.5 / 12.6, 2960: 10.5 / 13.6, 6048: 16.7 / 14.6; P = 2 Roe 1404:
+// 10.5 / 12.6, 2520: 14.6 / 12.6; quads of P = 3 Euler, 5850: 16.7 / 18.7, 8188:
+// 20.8 / 19.1.
+template <int D, int NU, int NF>
+MixedKernels mixed_kernels_for(long long E, int pf)
+{
+  constexpr bool doubles = shape_epb(kUpdShapes[1], NF, true) <= 2 * kUpdShapes[1].epb;
+  const int per_sm = pf == 0 ? 3 : (pf == 2 ? 4 : (doubles ? 10 : 5));
+  return E > 4LL * 148 * per_sm ? mixed_kernels<D, NU, NF, true>() : mixed_kernels<D, NU, NF, false>();
+}
+
 // the kernels of the 2-D element types of orders 2 and 3 (fr_mixed_fused_2d.cu)
-bool find_kernels_2d(int NU, int NF, MixedKernels* out);
+bool find_kernels_2d(int NU, int NF, long long E, int pf, MixedKernels* out);
 // the kernels of orders 1 and 4 (fr_mixed_fused_p14.cu)
-bool find_kernels_p14(int D, int NU, int NF, MixedKernels* out);
+bool find_kernels_p14(int D, int NU, int NF, long long E, int pf, MixedKernels* out);
 
 }  // namespace frb_mixed

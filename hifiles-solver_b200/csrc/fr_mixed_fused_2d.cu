@@ -5,11 +5,11 @@
 
 namespace frb_mixed {
 
-bool find_kernels_2d(int NU, int NF, MixedKernels* out)
+bool find_kernels_2d(int NU, int NF, long long E, int pf, MixedKernels* out)
 {
 #define FR_MIXED_SHAPE(nu, nf) \
   if (NU == nu && NF == nf) {  \
-    *out = mixed_kernels<2, nu, nf>(); \
+    *out = mixed_kernels_for<2, nu, nf>(E, pf); \
     return true;               \
   }
   FR_MIXED_SHAPE(6, 9)    // triangle P2

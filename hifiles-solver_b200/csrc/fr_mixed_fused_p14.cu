@@ -7,11 +7,11 @@
 
 namespace frb_mixed {
 
-bool find_kernels_p14(int D, int NU, int NF, MixedKernels* out)
+bool find_kernels_p14(int D, int NU, int NF, long long E, int pf, MixedKernels* out)
 {
 #define FR_MIXED_SHAPE(d, nu, nf)          \
   if (D == d && NU == nu && NF == nf) {    \
-    *out = mixed_kernels<d, nu, nf>();     \
+    *out = mixed_kernels_for<d, nu, nf>(E, pf); \
     return true;                           \
   }
   FR_MIXED_SHAPE(3, 4, 12)    // tet P1

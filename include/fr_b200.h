@@ -733,12 +733,15 @@ fr_status fr_mixed_stage_advance(fr_mixed_stage* s, int n_steps, double dt, void
  * Synchronises the stream; FR_ERR_NONFINITE for a NaN norm. */
 fr_status fr_mixed_stage_advance_norms(fr_mixed_stage* s, int n_steps, double dt, double* res_norms, void* stream);
 /* Launch shapes of each type's two stage kernels: gradient 0 = 8 elements x
- * 256 threads, 1 = 4 x 128, 2 = 8 x 128, 3 = 4 x 128 with registers for 4
- * blocks per SM, 4 = 8 x 256 with registers for 2; update 0 = 8 x 256,
- * 1 = 4 x 128,
- * 2 = 8 x 128 (every shape gives the same bits; shapes whose shared memory
- * exceeds a block's return FR_ERR_UNSUPPORTED).  create() sets gradient 3
- * and update 1 (else the first shape that fits);
+ * 256 threads, 1 = 4 x 128 with registers for 3 blocks per SM, 2 = 4 x 160
+ * for 3, 3 = 4 x 128 for 4, 4 = 8 x 256 for 2; update 0 = 8 x 256 for 2,
+ * 1 = 4 x 160 for 3, 2 = 4 x 128 for 4 (every shape gives the same bits;
+ * shapes whose shared memory exceeds a block's return FR_ERR_UNSUPPORTED; the
+ * Euler forms have gradient 1 and update 1 only).  Types with few flux points
+ * take more elements per block, as many as give each flux point a thread: in
+ * gradient 3, update 1 and the Euler forms where the mesh is large enough to
+ * fill the GPU with such blocks, in the other shapes always.  create() sets
+ * gradient 3 and update 1 (else the first shape that fits);
  * autotune() times every shape on the current state (the update kernels in
  * residual mode, into scratch memory; the state is not changed) and keeps
  * the fastest per type. */

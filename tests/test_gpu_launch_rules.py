@@ -118,3 +118,61 @@ def test_mixed_norms_do_not_depend_on_the_launch_shape(P, viscous):
     for nrm, st in out:
         assert np.all(nrm > 0) and np.array_equal(st, out[0][1])
         assert np.all(np.abs(nrm - out[0][0]) <= 1e-12 * out[0][0])
+
+
+def _box_2d(kind, nx, ny, x1):
+    """Vertices and cells of the box [0, x1] x [0, 10], nx x ny quads or pairs of triangles, row by row."""
+    from hifiles_b200 import mixed as X
+    xv = np.stack([a.ravel() for a in np.meshgrid(np.linspace(0, x1, nx + 1), np.linspace(0, 10, ny + 1))], axis=1)
+    cells = []
+    for j in range(ny):
+        for i in range(nx):
+            a, d = i + (nx + 1) * j, i + (nx + 1) * (j + 1)
+            if kind == X.QUAD:
+                cells.append((X.QUAD, (a, a + 1, d, d + 1)))
+            else:
+                cells += [(X.TRI, (a, a + 1, d + 1)), (X.TRI, (a, d + 1, d))]
+    return xv, cells
+
+
+# cells of the smaller mesh: at most 4 x 148 elements times 3 blocks per SM
+# (Navier-Stokes), 5 (Euler; 10 where a block's elements only double) or 4 (Roe)
+@pytest.mark.parametrize("kind,P,form,n", [
+    ("tri", 1, "ns", (29, 30)), ("tri", 2, "ns", (29, 30)), ("tri", 3, "ns", (29, 30)), ("tri", 4, "ns", (29, 30)),
+    ("tri", 1, "euler", (40, 37)), ("tri", 2, "euler", (40, 37)), ("tri", 3, "euler", (40, 37)),
+    ("tri", 4, "euler", (54, 54)), ("tri", 2, "roe", (37, 32)), ("tri", 4, "roe", (37, 32)),
+    ("quad", 1, "ns", (42, 42)), ("quad", 2, "ns", (42, 42)), ("quad", 3, "ns", (42, 42)), ("quad", 4, "ns", (42, 42)),
+    ("quad", 1, "euler", (54, 54)), ("quad", 2, "euler", (54, 54)), ("quad", 3, "euler", (76, 77)),
+    ("quad", 4, "euler", (76, 77)), ("quad", 2, "roe", (48, 49)), ("quad", 3, "roe", (48, 49))])
+def test_elements_per_block_do_not_change_the_state(kind, P, form, n):
+    """A mesh below the size where the mixed stage's blocks are filled, and two
+    copies of it side by side, above: each copy of a periodic state advances as
+    the small mesh does.  The copies' coordinates differ from the original's in
+    their last bits (20 / 0.13 eps of a cell's size, 4e-14), and so by less than
+    1e-12 the states."""
+    from hifiles_b200 import mixed as X
+    from hifiles_b200 import seam
+    t = X.TRI if kind == "tri" else X.QUAD
+    cells = n[0] * n[1] * (2 if kind == "tri" else 1)
+    most = 4 * 148 * {"ns": 3, "euler": 10 if P >= 4 or (kind == "quad" and P == 3) else 5, "roe": 4}[form]
+    assert cells <= most < 2 * cells
+    phys = dict(gamma=1.4, prandtl=0.71, mu_inf=1e-2, rt_inf=1.0, c_sth=1.0, fix_vis=1.0, tau=1.0, pen_fact=0.5)
+    out = []
+    for k in (1, 2):
+        xv, c = _box_2d(t, k * n[0], n[1], 10.0 * k)
+        mesh = X.MixedMesh(P, xv, c, np.array([10.0 * k, 10.0]), (), X.ElementOpts(vcjh_scheme_tri=1))
+        pos = mesh.types[t]["pos_upts"]
+        x, y = 0.2 * np.pi * pos[..., 0], 0.2 * np.pi * pos[..., 1]
+        rho, u, v = 1 + 0.1 * np.sin(x) * np.cos(y), 0.5 + 0.1 * np.cos(y), 0.2 * np.sin(x + y)
+        p = 1 + 0.05 * np.cos(x - y)
+        u0 = np.asfortranarray(np.stack([rho, rho * u, rho * v, p / 0.4 + 0.5 * rho * (u * u + v * v)], axis=-1))
+        types, ints, bdys = mesh.operator_inputs({t: u0})
+        m = seam.FusedMixedMesh(types, ints, phys, bdys, viscous=form == "ns", riemann=2 if form == "roe" else 0)
+        nrm = m.advance(3, 1e-3, norms=True)
+        out.append((m.get_state(t), nrm, u0))
+    (a, na, u0), (b, nb, _) = out
+    per = 2 if kind == "tri" else 1
+    row = b.reshape(b.shape[0], n[1], 2 * n[0] * per, 4)    # elements row by row
+    assert rel(a, u0) > 1e-5 and np.all(np.abs(nb - na) <= 1e-9 * na)
+    for copy in (row[:, :, :n[0] * per], row[:, :, n[0] * per:]):
+        assert rel(copy.reshape(a.shape), a) <= 1e-12
