@@ -335,6 +335,7 @@ __device__ __noinline__ void vis_boundary(PhysT<TC> ph, int type, BdyPoint<D, TC
 //   oG   reference gradient, then in place the physical gradient [F*D]
 //   oUf  own solution at the flux points [F][element][NF]
 //   oS   transformed SGS flux [(F-1)*D] (LES only)
+//   oMlp the learned closure's parameters (LES 2 only)
 // Region sizes are rounded up to 4 words: every region starts on 16 bytes.
 template <int DIM, int P, int EPB, typename TC>
 struct GradPlan {
@@ -345,12 +346,13 @@ struct GradPlan {
   static constexpr int oDJ = oM + r4(EPB * DIM * DIM * S::NU), oG = oDJ + r4(EPB * S::NU);
   static constexpr int oUf = oG + r4(S::F * DIM * NW), oS = oUf + r4(S::F * EPB * S::NF);
   __host__ __device__ static constexpr int size(int les) { return oS + (les ? r4((S::F - 1) * DIM * NW) : 0); }
+  static constexpr int oMlp = (int)sizeof(TC) * size(1);   // in bytes
 };
 
 template <int DIM, int P, int EPB, typename TC, int LES = 0>
 __host__ __device__ constexpr size_t grad_smem_bytes()
 {
-  return sizeof(TC) * GradPlan<DIM, P, EPB, TC>::size(LES);
+  return sizeof(TC) * GradPlan<DIM, P, EPB, TC>::size(LES) + (LES == 2 ? kMlpSmem : 0);
 }
 
 // Viscous stage, part 1 (per element):
@@ -365,8 +367,8 @@ __host__ __device__ constexpr size_t grad_smem_bytes()
 //   gradient (what calculate_common_viscFlux evaluates for this side), kept
 //   only as its projection on the interface's left normal: VF (F-1 values,
 //   the mass component is zero).
-// With LES = 1 the eddy-viscosity SGS flux joins the viscous flux at the
-// solution points (evaluate_viscFlux, src/eles.cpp:2369-2380); its transformed
+// With LES = 1 the eddy-viscosity SGS flux (Smagorinsky, WALE), with LES = 2 the
+// learned closure's, joins the viscous flux at the solution points (evaluate_viscFlux, src/eles.cpp:2369-2380); its transformed
 // components (sgsf_upts, src/eles.cpp:2382-2409) are extrapolated to the flux
 // points (evaluate_sgsFlux, src/eles.cpp:3294-3368) and added there to the
 // physical viscous flux before the projection, as calculate_common_viscFlux
@@ -428,6 +430,8 @@ fr_grad_body(long long blk0, long long bstride, const double* __restrict__ U, co
   auto grad = [&](int k, int d, int el) { return sG + (k + F * d) * NW + el * M::N; };
   const int tid = threadIdx.x;
   const long long NFE = (long long)NF * E;
+  // the closure's parameters, waited for with the state
+  if constexpr (LES == 2) cp_run<4, NT>(reinterpret_cast<float*>(fr_smem + G::oMlp), ph.mlp, kMlpN);
   // the thread's line task
   const int k = tid / (EPB * NLN), kr = tid - k * (EPB * NLN), el = kr / NLN, j = kr - el * NLN;
   const int j0 = DIM == 3 ? j % N1 : j, j1 = DIM == 3 ? j / N1 : 0;
@@ -600,7 +604,8 @@ fr_grad_body(long long blk0, long long bstride, const double* __restrict__ U, co
     for (int m = 0; m < DD; m++) g[m] = gj[m];
     if constexpr (LES != 0) {
       TC fs[F][D];
-      sgs_flux<D, TC>(ph, q, gp, dj, TC(P + 1), fs);
+      if constexpr (LES == 2) sgs_flux_learned<D, TC>(G::oMlp, ph.gamma, q, gp, dj, TC(P + 1), ph.filter_ratio, fs);
+      else sgs_flux<D, TC>(ph, q, gp, dj, TC(P + 1), fs);
 #pragma unroll
       for (int kk = 1; kk < F; kk++)
 #pragma unroll

@@ -55,6 +55,53 @@ __device__ __forceinline__ float mlp_eval(const float* __restrict__ w, const flo
   return mlp_softplus(o);
 }
 
+// The same for the stage kernels, from a copy of the parameters in the block's
+// dynamic shared memory (byte offset off, 16-byte aligned).  A stage runs few
+// blocks per SM, whose registers are capped (80 to 128) and whose shared memory
+// leaves little of the L1 cache: every weight read through it was a round trip,
+// many of them to L2, with few in flight.  Out of line, so that a point's state
+// and gradient are saved once around it; kMlpRows rows of W2 at a time, so that
+// as many sums are in flight and a load brings four weights.  Every sum is taken
+// in the order of mlp_eval: same bits.
+constexpr int kMlpRows = 4;
+constexpr int kMlpSmem = (kMlpN * 4 + 15) / 16 * 16;
+struct MlpInputs {
+  float x[kMlpIn];
+};
+static __device__ __noinline__ float mlp_eval_shared(int off, MlpInputs in)
+{
+  extern __shared__ __align__(16) unsigned char fr_smem[];
+  const float* w = reinterpret_cast<const float*>(fr_smem + off);
+  float h1[kMlpH];
+#pragma unroll
+  for (int k = 0; k < kMlpIn; k++) in.x[k] = (in.x[k] - w[kMlpXm + k]) * w[kMlpXs + k];
+#pragma unroll
+  for (int i = 0; i < kMlpH; i++) {
+    float a = w[kMlpB1 + i];
+#pragma unroll
+    for (int k = 0; k < kMlpIn; k++) a = fmaf(w[kMlpW1 + i * kMlpIn + k], in.x[k], a);
+    h1[i] = tanhf(a);
+  }
+  float o = w[kMlpB3];
+  for (int j = 0; j < kMlpH; j += kMlpRows) {
+    float a[kMlpRows];
+#pragma unroll
+    for (int r = 0; r < kMlpRows; r++) a[r] = w[kMlpB2 + j + r];
+#pragma unroll
+    for (int i = 0; i < kMlpH; i += 4) {
+      float4 v[kMlpRows];
+#pragma unroll
+      for (int r = 0; r < kMlpRows; r++) v[r] = *reinterpret_cast<const float4*>(w + kMlpW2 + (j + r) * kMlpH + i);
+#pragma unroll
+      for (int r = 0; r < kMlpRows; r++)
+        a[r] = fmaf(v[r].w, h1[i + 3], fmaf(v[r].z, h1[i + 2], fmaf(v[r].y, h1[i + 1], fmaf(v[r].x, h1[i], a[r]))));
+    }
+#pragma unroll
+    for (int r = 0; r < kMlpRows; r++) o = fmaf(w[kMlpW3 + j + r], tanhf(a[r]), o);
+  }
+  return mlp_softplus(o);
+}
+
 // Inputs of the closure at one point from the conserved state q and its
 // physical gradient g[k][l] = d q_k / d x_l.  With A_ij = d u_i / d x_j,
 // S the deviatoric symmetric part and W the antisymmetric part of A, and
@@ -136,15 +183,16 @@ __device__ __forceinline__ void sgs_learned_inputs(const T* q, const T (*g)[D], 
 
 // SGS flux of the learned closure: mu_t = rho Delta^2 |S| c(x); momentum
 // -2 mu_t S, energy -gamma mu_t / 0.5 de (the flux form of calc_sgsf_upts).
+// off: the parameters' place in the block's shared memory (mlp_eval_shared).
 template <int D, typename T>
-__device__ __forceinline__ void sgs_flux_learned(const float* __restrict__ w, T gamma, const T* q, const T (*g)[D],
+__device__ __forceinline__ void sgs_flux_learned(int off, T gamma, const T* q, const T (*g)[D],
                                                  T detjac, T n1, T filter_ratio, T (*fs)[D])
 {
   constexpr int F = D + 2;
-  float x[kMlpIn];
+  MlpInputs in;
   T delta, S[D][D], smag, de[D];
-  sgs_learned_inputs<D, T>(q, g, detjac, n1, filter_ratio, x, delta, S, smag, de);
-  const T c = (T)mlp_eval(w, x);
+  sgs_learned_inputs<D, T>(q, g, detjac, n1, filter_ratio, in.x, delta, S, smag, de);
+  const T c = (T)mlp_eval_shared(off, in);
   const T mu_t = q[0] * delta * delta * smag * c;
 #pragma unroll
   for (int j = 0; j < D; j++) {

@@ -602,7 +602,7 @@ __device__ __forceinline__ void ldg_flux(const PhysT<T>& ph, T pen, const T* ul,
 // WALE, Cw = 0.5; no wall model; src/eles.cpp:2456-2778), physical
 // components fs[k][l].  g is the physical gradient g[k][l] = d q_k / d x_l,
 // detjac the Jacobian determinant at the point, n1 = order + 1.
-// sgs_model 5 is the learned closure of fr_mlp.cuh (no reference counterpart).
+// (sgs_model 5, the learned closure, is sgs_flux_learned of fr_mlp.cuh.)
 //
 // Two index choices of the reference are kept as it evaluates them: its
 // "velocity" vector is u_i = q_i / rho for i < D, so u_0 = rho / rho
@@ -617,10 +617,6 @@ template <int D, typename T>
 __device__ __forceinline__ void sgs_flux(const PhysT<T>& ph, const T* q, const T (*g)[D], T detjac, T n1,
                                          T (*fs)[D])
 {
-  if (ph.sgs_model == 5) {
-    sgs_flux_learned<D, T>(ph.mlp, ph.gamma, q, g, detjac, n1, ph.filter_ratio, fs);
-    return;
-  }
   constexpr int F = D + 2;
   const T rho = q[0];
   T u[D], ke = T(0);

@@ -162,8 +162,9 @@ struct RunnerT : Runner {
   }
   void grad(const Bufs& b, int cur, cudaStream_t s) override
   {
-    if (les) grad_i<0, 1>(b, cur, s);
-    else grad_i<0, 0>(b, cur, s);
+    if (!les) grad_i<0, 0>(b, cur, s);
+    else if (ph.sgs_model == 5) grad_i<0, 2>(b, cur, s);
+    else grad_i<0, 1>(b, cur, s);
   }
 
   template <int VISC>

@@ -22,11 +22,16 @@ NS = dict(gamma=1.4, prandtl=0.71, mu_inf=1e-3, tau=1.0, pen_fact=0.5)
 @pytest.mark.parametrize("dims,P,n", [(2, 1, (5, 7)), (2, 2, (3, 7)), (2, 3, (5, 5)), (2, 4, (7, 3)), (2, 5, (3, 5)),
                                       (3, 1, (3, 5, 3)), (3, 2, (3, 3, 3)), (3, 3, (1, 3, 1)), (3, 4, (1, 1, 1)),
                                       (3, 4, (3, 1, 3))])
-@pytest.mark.parametrize("form", ["ns", "euler", "fp32", "wale"])
+@pytest.mark.parametrize("form", ["ns", "euler", "fp32", "wale", "learned"])
 def test_every_tile_gives_the_same_state(dims, P, n, form):
     visc = form != "euler"
     s = H.Solver.box(dims, P, n, [0.0] * dims, [2 * np.pi] * dims, jitter=0.1, seed=5, viscous=visc,
-                     precision=int(form == "fp32"), les=int(form == "wale"), sgs_model=1, **NS)
+                     precision=int(form == "fp32"), les=int(form in ("wale", "learned")),
+                     sgs_model=5 if form == "learned" else 1, **NS)
+    if form == "learned":            # weights that matter: c near softplus(-1)
+        w = M.init_params(5)
+        w[M.B3] = -1.0
+        s.set_sgs_mlp(w)
     pos = s.geometry()["pos_upts"]
     u0 = O.ic_tgv(pos) if dims == 3 else O.ic_vortex(pos * (10 / (2 * np.pi)) - 5)
     s.set_state(u0)
