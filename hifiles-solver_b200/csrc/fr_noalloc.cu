@@ -72,7 +72,7 @@ template <> struct NaTile<2, 1> { static constexpr int EPB = 16, NT = 128; };
 template <> struct NaTile<2, 2> { static constexpr int EPB = 10, NT = 128; };
 template <> struct NaTile<2, 3> { static constexpr int EPB = 8, NT = 128; };
 template <> struct NaTile<2, 4> { static constexpr int EPB = 5, NT = 128; };
-template <> struct NaTile<2, 5> { static constexpr int EPB = 5, NT = 192; };
+template <> struct NaTile<2, 5> { static constexpr int EPB = 3, NT = 128; };
 template <> struct NaTile<3, 1> { static constexpr int EPB = 6, NT = 160; };
 template <> struct NaTile<3, 2> { static constexpr int EPB = 4, NT = 224; };
 template <> struct NaTile<3, 3> { static constexpr int EPB = 2, NT = 192; };
