@@ -356,8 +356,11 @@ fr_status fr_mixed_stage_create(int n_dims, int n_types, const fr_mixed_stage_ty
                                                 " solution / " + std::to_string(NF) + " flux points"));
     s->kern.push_back(k);
     // defaults before any autotune: the shapes that measured fastest for
-    // tets (4 elements x 128 threads), else the first that fits
+    // tets (4 elements x 128 threads, registers for four blocks per SM; for
+    // three where an SM's shared memory holds a single block, as of hexes of
+    // P = 3: 576 of them 53.6 us a stage against 57.8), else the first that fits
     int g0 = 3, u0 = 1;
+    if (pf == 0 && 2 * (k.smem_a[0][3] + 1024) > 228 * 1024) g0 = 1;
     if (!k.grad[pf][g0])
       for (g0 = 0; g0 < kNGrad - 1 && !k.grad[pf][g0];) g0++;
     if (!k.upd1[pf][u0])

@@ -741,7 +741,8 @@ fr_status fr_mixed_stage_advance_norms(fr_mixed_stage* s, int n_steps, double dt
  * take more elements per block, as many as give each flux point a thread: in
  * gradient 3, update 1 and the Euler forms where the mesh is large enough to
  * fill the GPU with such blocks, in the other shapes always.  create() sets
- * gradient 3 and update 1 (else the first shape that fits);
+ * gradient 3 (1 for types whose blocks fill an SM's shared memory, hexes of
+ * order 3 for instance) and update 1 (else the first shape that fits);
  * autotune() times every shape on the current state (the update kernels in
  * residual mode, into scratch memory; the state is not changed) and keeps
  * the fastest per type. */

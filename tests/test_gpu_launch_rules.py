@@ -125,6 +125,20 @@ def test_mixed_norms_do_not_depend_on_the_launch_shape(P, viscous):
         assert np.all(np.abs(nrm - out[0][0]) <= 1e-12 * out[0][0])
 
 
+@pytest.mark.parametrize("P,shape", [(1, (3, 1)), (2, (3, 1)), (3, (1, 1))])
+def test_mixed_stage_default_shapes(P, shape):
+    """Registers for four blocks per SM where more than one fits its shared memory."""
+    from hifiles_b200 import mixed as X
+    from hifiles_b200 import seam
+    xv, c2v = H.box_mesh(3, (3, 3, 2), (0, 0, 0), (1, 1, 1))
+    mesh = X.MixedMesh(P, xv, [(X.HEX, tuple(int(v) for v in c)) for c in c2v], np.array([1.0] * 3), (), X.ElementOpts())
+    u0 = np.zeros(mesh.types[X.HEX]["pos_upts"].shape[:2] + (5,), order="F")
+    u0[..., 0], u0[..., 4] = 1.0, 2.5
+    types, ints, bdys = mesh.operator_inputs({X.HEX: u0})
+    m = seam.FusedMixedMesh(types, ints, dict(NS, rt_inf=1.0, c_sth=1.0, fix_vis=1.0), bdys)
+    assert tuple(m.launch(X.HEX)) == shape
+
+
 def _box_2d(kind, nx, ny, x1):
     """Vertices and cells of the box [0, x1] x [0, 10], nx x ny quads or pairs of triangles, row by row."""
     from hifiles_b200 import mixed as X
