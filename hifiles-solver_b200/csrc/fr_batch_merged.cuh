@@ -2,16 +2,16 @@
 //
 // A batch holds one merged mesh per (order, scheme) group.  Run group by
 // group, a viscous RK stage launches the gradient kernel, the interface-flux
-// kernel (orders whose runs are not 16-byte multiples) and the update kernel
-// of every group: 2-3 launches per group and stage.  The merged launches
+// kernel (orders 2 and 4) and the update kernel of every group: 2-3 launches
+// per group and stage.  The merged launches
 // below run each of those kernels once for all groups of hexahedra of orders
 // 2, 3 and 4: the grid is the concatenation of the groups' element blocks,
 // and each block runs the body of its group's order on that group's buffers
 // (one body per block, chosen by the block index, so every barrier of a body
 // is reached by the whole block).  All groups use blocks of 192 threads with
-// as many elements as give each flux point a thread; order 3 takes the fused interface/update body, orders 2 and 4
-// the interface-flux and update bodies.  No norms are formed (the batch reports
-// none).
+// as many elements as give each flux point a thread; order 3 takes the fused
+// interface/update body, orders 2 and 4 the interface-flux and update bodies.
+// No norms are formed (the batch reports none).
 #pragma once
 
 #include "fr_b200.h"
@@ -19,8 +19,13 @@
 
 namespace frb {
 
-// threads per block and elements per block: 162, 192 and 150 of 192 threads
-// have a flux point
+// Threads per block and elements per block: 162, 192 and 150 of 192 threads
+// have a flux point.  The cap for four CTAs per SM spills (FP64 gradient kernel,
+// 80 registers: 1.6 kB of stores), yet is the fastest: a step of 12 boxes of
+// 6^3 to 14^3, us, caps for 4 / 3 / 1 CTAs: 1545 / 1649 / 1771, FP32 1041 / 1128 /
+// 1357; of 6 boxes of 4^3 to 6^3 130 / 139 / 145.  Blocks of 128 threads (2, 1 and
+// 1 elements) spill a fifth of that and take 1570 / 1703 / 1688, FP32 1057 / 1142 /
+// 1143; 133 / 158 / 157.  Per-group launches: 1370, 1030; 203.
 constexpr int kMergedNT = 192;
 template <int P> struct MergedTile { static constexpr int epb = P == 2 ? 3 : P == 3 ? 2 : 1; };
 

@@ -6,8 +6,9 @@
 // interpolated to each cubature point with the dense nodal-basis rows
 // opp_volume_cubpts (column order, as the reference's loop), the quantities
 // are formed with the reference's expressions, and weight x detJ at the
-// cubature point integrates them.  Per-block partial sums, added by fr_diag_finalize in a fixed order, so the
-// result does not depend on scheduling.
+// cubature point integrates them.  Per-block partial sums, added by
+// fr_diag_finalize in a fixed order, so the result does not depend on
+// scheduling.
 #include <cuda_runtime.h>
 
 namespace frb {
@@ -30,7 +31,10 @@ __host__ __device__ inline int diag_ld(int nu)
   while (x % 16 != 4 && x % 16 != 12) x++;
   return x;
 }
-inline size_t diag_smem(int nu, int cols) { return sizeof(double) * (size_t)((cols + 7) / 8 * 8) * (diag_ld(nu) + kDiagLdv); }
+inline size_t diag_smem(int nu, int cols)
+{
+  return sizeof(double) * (size_t)((cols + 7) / 8 * 8) * (diag_ld(nu) + kDiagLdv);
+}
 
 // largest dynamic shared memory of a block: the device's 227 KB less the
 // kernel's own norm partials
@@ -90,118 +94,118 @@ fr_diag_kernel(const double* __restrict__ U, const TG* __restrict__ G, const dou
     }
     __syncthreads();
     for (int j0 = kDiagRows * blockIdx.y; j0 < nc; j0 += kDiagRows * gridDim.y) {
-    const int rows = nc - j0 < kDiagRows ? nc - j0 : kDiagRows;
-    const int MT = (rows + 7) / 8, NB = (NTL + kDiagTN - 1) / kDiagTN;
-    for (int u = warp; u < MT * NB; u += kDiagWarps) {
-      const int mt = u / NB, nt0 = (u - mt * NB) * kDiagTN, r = j0 + mt * 8 + g8;
-      double c[kDiagTN][2];
-      const double* bp[kDiagTN];
+      const int rows = nc - j0 < kDiagRows ? nc - j0 : kDiagRows;
+      const int MT = (rows + 7) / 8, NB = (NTL + kDiagTN - 1) / kDiagTN;
+      for (int u = warp; u < MT * NB; u += kDiagWarps) {
+        const int mt = u / NB, nt0 = (u - mt * NB) * kDiagTN, r = j0 + mt * 8 + g8;
+        double c[kDiagTN][2];
+        const double* bp[kDiagTN];
 #pragma unroll
-      for (int j = 0; j < kDiagTN; j++) {
-        c[j][0] = c[j][1] = 0.0;
-        bp[j] = sB + (size_t)((nt0 + j < NTL ? nt0 + j : nt0) * 8 + g8) * ldk + t4;
-      }
-      for (int k0 = 0; k0 < KS; k0 += 8) {
-        double a[8];
+        for (int j = 0; j < kDiagTN; j++) {
+          c[j][0] = c[j][1] = 0.0;
+          bp[j] = sB + (size_t)((nt0 + j < NTL ? nt0 + j : nt0) * 8 + g8) * ldk + t4;
+        }
+        for (int k0 = 0; k0 < KS; k0 += 8) {
+          double a[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int k = (k0 + i) * 4 + t4;
-          a[i] = (r < nc && k < nu) ? __ldg(opp + r + (size_t)nc * k) : 0.0;
+          for (int i = 0; i < 8; i++) {
+            const int k = (k0 + i) * 4 + t4;
+            a[i] = (r < nc && k < nu) ? __ldg(opp + r + (size_t)nc * k) : 0.0;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            if (k0 + i < KS)
+#pragma unroll
+              for (int j = 0; j < kDiagTN; j++)
+                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                    : "+d"(c[j][0]), "+d"(c[j][1])
+                    : "d"(a[i]), "d"(bp[j][(k0 + i) * 4]));
         }
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-          if (k0 + i < KS)
-#pragma unroll
-            for (int j = 0; j < kDiagTN; j++)
-              asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                  : "+d"(c[j][0]), "+d"(c[j][1])
-                  : "d"(a[i]), "d"(bp[j][(k0 + i) * 4]));
+        for (int j = 0; j < kDiagTN; j++)
+          if (nt0 + j < NTL) {
+            double* v = sV + (size_t)((nt0 + j) * 8 + 2 * t4) * kDiagLdv + mt * 8 + g8;
+            v[0] = c[j][0];
+            v[kDiagLdv] = c[j][1];
+          }
       }
+      __syncthreads();
+      for (int i = tid; i < nval * rows; i += kDiagThreads) {
+        const int el = i / rows, jj = i - el * rows, j = j0 + jj;
+        const long long e = e0 + el;
+        const double* v = sV + (size_t)el * C * kDiagLdv + jj;
+        double u[F], g[F][D];
 #pragma unroll
-      for (int j = 0; j < kDiagTN; j++)
-        if (nt0 + j < NTL) {
-          double* v = sV + (size_t)((nt0 + j) * 8 + 2 * t4) * kDiagLdv + mt * 8 + g8;
-          v[0] = c[j][0];
-          v[kDiagLdv] = c[j][1];
+        for (int m = 0; m < F; m++) {
+          u[m] = v[m * kDiagLdv];
+          if constexpr (NQ > 1) {
+#pragma unroll
+            for (int n = 0; n < D; n++) g[m][n] = v[(F + m + F * n) * kDiagLdv];
+          }
         }
-    }
-    __syncthreads();
-    for (int i = tid; i < nval * rows; i += kDiagThreads) {
-    const int el = i / rows, jj = i - el * rows, j = j0 + jj;
-    const long long e = e0 + el;
-    const double* v = sV + (size_t)el * C * kDiagLdv + jj;
-    double u[F], g[F][D];
+        const double wj = W[j], dj = detj[j + (size_t)nc * e];
+        const double irho = 1. / u[0];
+        double tke = 0.0;
 #pragma unroll
-    for (int m = 0; m < F; m++) {
-      u[m] = v[m * kDiagLdv];
-      if constexpr (NQ > 1) {
+        for (int n = 1; n < F - 1; n++) tke += 0.5 * u[n] * u[n];
+        acc[0] += irho * tke * wj * dj;
+        if constexpr (NQ > 1) {
+          const double dudx = irho * (g[1][0] - u[1] * irho * g[0][0]);
+          const double dudy = irho * (g[1][1] - u[1] * irho * g[0][1]);
+          const double dvdx = irho * (g[2][0] - u[2] * irho * g[0][0]);
+          const double dvdy = irho * (g[2][1] - u[2] * irho * g[0][1]);
+          double dudz = 0, dvdz = 0, dwdx = 0, dwdy = 0, dwdz = 0;
+          if (D == 3) {
+            dudz = irho * (g[1][D - 1] - u[1] * irho * g[0][D - 1]);
+            dvdz = irho * (g[2][D - 1] - u[2] * irho * g[0][D - 1]);
+            dwdx = irho * (g[D][0] - u[D] * irho * g[0][0]);
+            dwdy = irho * (g[D][1] - u[D] * irho * g[0][1]);
+            dwdz = irho * (g[D][D - 1] - u[D] * irho * g[0][D - 1]);
+          }
+          // vorticity: rho |w|^2 / 2
+          const double wz = dvdx - dudy;
+          double vort = wz * wz;
+          if (D == 3) {
+            const double wx = dwdy - dvdz, wy = dudz - dwdx;
+            vort += wx * wx + wy * wy;
+          }
+          vort *= 0.5 / irho;
+          // pressure dilatation
+          const double pressure = (gamma - 1.0) * (u[F - 1] - irho * tke);
+          const double pd = D == 2 ? pressure * (dudx + dvdy) : pressure * (dudx + dvdy + dwdz);
+          // strain-rate colon products
+          double S[3][3];
+          S[0][0] = dudx;
+          S[0][1] = (dudy + dvdx) / 2.0;
+          S[1][0] = S[0][1];
+          S[1][1] = dvdy;
+          double diag = (S[0][0] + S[1][1]) / 3.0;
+          if (D == 3) {
+            S[0][2] = (dudz + dwdx) / 2.0;
+            S[1][2] = (dvdz + dwdy) / 2.0;
+            S[2][0] = S[0][2];
+            S[2][1] = S[1][2];
+            S[2][2] = dwdz;
+            diag += S[2][2] / 3.0;
+          }
+          double sc = 0.0, dsc = 0.0;
 #pragma unroll
-        for (int n = 0; n < D; n++) g[m][n] = v[(F + m + F * n) * kDiagLdv];
+          for (int a = 0; a < D; a++)
+#pragma unroll
+            for (int b = 0; b < D; b++) sc += S[a][b] * S[a][b];
+#pragma unroll
+          for (int a = 0; a < D; a++) S[a][a] -= diag;
+#pragma unroll
+          for (int a = 0; a < D; a++)
+#pragma unroll
+            for (int b = 0; b < D; b++) dsc += S[a][b] * S[a][b];
+          acc[1] += vort * wj * dj;
+          acc[2 % NQ] += pd * wj * dj;
+          acc[3 % NQ] += sc * wj * dj;
+          acc[4 % NQ] += dsc * wj * dj;
+        }
       }
-    }
-    const double wj = W[j], dj = detj[j + (size_t)nc * e];
-    const double irho = 1. / u[0];
-    double tke = 0.0;
-#pragma unroll
-    for (int n = 1; n < F - 1; n++) tke += 0.5 * u[n] * u[n];
-    acc[0] += irho * tke * wj * dj;
-    if constexpr (NQ > 1) {
-      const double dudx = irho * (g[1][0] - u[1] * irho * g[0][0]);
-      const double dudy = irho * (g[1][1] - u[1] * irho * g[0][1]);
-      const double dvdx = irho * (g[2][0] - u[2] * irho * g[0][0]);
-      const double dvdy = irho * (g[2][1] - u[2] * irho * g[0][1]);
-      double dudz = 0, dvdz = 0, dwdx = 0, dwdy = 0, dwdz = 0;
-      if (D == 3) {
-        dudz = irho * (g[1][D - 1] - u[1] * irho * g[0][D - 1]);
-        dvdz = irho * (g[2][D - 1] - u[2] * irho * g[0][D - 1]);
-        dwdx = irho * (g[D][0] - u[D] * irho * g[0][0]);
-        dwdy = irho * (g[D][1] - u[D] * irho * g[0][1]);
-        dwdz = irho * (g[D][D - 1] - u[D] * irho * g[0][D - 1]);
-      }
-      // vorticity: rho |w|^2 / 2
-      const double wz = dvdx - dudy;
-      double vort = wz * wz;
-      if (D == 3) {
-        const double wx = dwdy - dvdz, wy = dudz - dwdx;
-        vort += wx * wx + wy * wy;
-      }
-      vort *= 0.5 / irho;
-      // pressure dilatation
-      const double pressure = (gamma - 1.0) * (u[F - 1] - irho * tke);
-      const double pd = D == 2 ? pressure * (dudx + dvdy) : pressure * (dudx + dvdy + dwdz);
-      // strain-rate colon products
-      double S[3][3];
-      S[0][0] = dudx;
-      S[0][1] = (dudy + dvdx) / 2.0;
-      S[1][0] = S[0][1];
-      S[1][1] = dvdy;
-      double diag = (S[0][0] + S[1][1]) / 3.0;
-      if (D == 3) {
-        S[0][2] = (dudz + dwdx) / 2.0;
-        S[1][2] = (dvdz + dwdy) / 2.0;
-        S[2][0] = S[0][2];
-        S[2][1] = S[1][2];
-        S[2][2] = dwdz;
-        diag += S[2][2] / 3.0;
-      }
-      double sc = 0.0, dsc = 0.0;
-#pragma unroll
-      for (int a = 0; a < D; a++)
-#pragma unroll
-        for (int b = 0; b < D; b++) sc += S[a][b] * S[a][b];
-#pragma unroll
-      for (int a = 0; a < D; a++) S[a][a] -= diag;
-#pragma unroll
-      for (int a = 0; a < D; a++)
-#pragma unroll
-        for (int b = 0; b < D; b++) dsc += S[a][b] * S[a][b];
-      acc[1] += vort * wj * dj;
-      acc[2 % NQ] += pd * wj * dj;
-      acc[3 % NQ] += sc * wj * dj;
-      acc[4 % NQ] += dsc * wj * dj;
-    }
-    }
-    __syncthreads();   // the values have been read
+      __syncthreads();   // the values have been read
     }
   }
 #pragma unroll
@@ -249,8 +253,8 @@ cudaError_t diag_launch(const double* U, const TG* G, const double* opp, const d
     return e;
   const long long groups = (E + epb - 1) / epb;
   // one block per group of elements over all its passes; a mesh of few groups
-  // spreads the passes of a large rule over more blocks (27 hexes of P = 3 with
-  // 1000 points: 80 us with 4 blocks of 32 passes)
+  // spreads the passes of a large rule over more blocks (kinetic energy of 27
+  // hexes of P = 3 with 729 points: 80 us with 4 blocks of 23 passes, 32 now)
   const int gx = (int)(groups < nblk ? groups : nblk), passes = (nc + kDiagRows - 1) / kDiagRows;
   const int gy = passes < nblk / gx ? passes : nblk / gx;
   fr_diag_kernel<D, TG, NQ><<<dim3(gx, gy), kDiagThreads, sm, st>>>(U, G, opp, W, detj, E, nu, nc, gamma, epb,

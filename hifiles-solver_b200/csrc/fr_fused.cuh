@@ -379,8 +379,9 @@ __host__ __device__ constexpr size_t grad_smem_bytes()
 // line's values are read once, its operator rows are compile-time entries of
 // the constant bank, and the element's fields fill F warps or more; the
 // pointwise fluxes are one solution point or flux point per thread, taking the
-// gradient one column at a time, so that 80 registers hold a point (a line's
-// two flux points per thread, and whole gradients, took 128).  Bound: FP64
+// gradient one column at a time, so that a point nearly fits 96 registers (FP64
+// P = 3: 40 bytes of spill stores; 224 at 80, none at 128 or in FP32; a line's
+// two flux points per thread, and whole gradients, filled 128).  Bound: FP64
 // issue, 60 k FP64 instructions per hex P = 3 element (948 cycles of an SM).
 // One output per thread instead, each reading its line and its operator row
 // from shared memory behind run-time index arithmetic, took 5.5 k warp

@@ -183,10 +183,11 @@ __device__ __forceinline__ void load_state(double* sU, const double* __restrict_
 }
 
 // ------------------------------------------------------------------ kernel A
-// A load phase issues every global read of the block (state, traces, the
-// neighbours' traces through mate, normals, metrics, wiring) into shared
-// memory, so the loads are in flight together; the compute phases that follow
-// touch global memory only to write.
+// A load phase issues the block's global reads together: state, own traces,
+// normals and metrics into shared memory, wiring and the neighbours' traces into
+// the registers of the threads that use them (blocks of more than four flux
+// points per thread read those where they use them, and boundary points their
+// place in the boundary list); otherwise the compute phases only write.
 template <int D, int NU, int NF, int EPB, int NTH, int MINB>
 __global__ void __launch_bounds__(NTH, MINB) mixed_grad_kernel(MixedType t, MixedFpts m,
                                                                const double* __restrict__ UFc, PhysT<double> ph)

@@ -259,7 +259,7 @@ int mma_ld(int k)
 
 size_t mma_smem(int k, int nb, int nct) { return (size_t)nb * nct * mma_ld(k) * sizeof(double); }
 
-// the column tile of every B_d fits one block's shared memory (128 columns, else 64)
+// a column tile of 64 columns of every B_d fits one block's shared memory
 bool mma_fits(int k, int nb) { return mma_smem(k, nb, 64) <= 200 * 1024; }
 
 fr_status dense_mma_launch(int m, int k, long long ncols, int nd, const OpSet& ops, const double* B, long long sB,
@@ -285,7 +285,7 @@ fr_status dense_mma_launch(int m, int k, long long ncols, int nd, const OpSet& o
               : nct == 128 ? pick(dense_mma_kernel<true, 128>, dense_mma_kernel<false, 128>)
               : nct == 64  ? pick(dense_mma_kernel<true, 64>, dense_mma_kernel<false, 64>)
                            : pick(dense_mma_kernel<true, 32>, dense_mma_kernel<false, 32>);
-  // every instantiation may use up to 100 kB: set once per device
+  // every instantiation may use what mma_fits lets through: set once per device
   static unsigned long long attr_set = 0;
   int dev = 0;
   cudaGetDevice(&dev);

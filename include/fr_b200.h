@@ -360,7 +360,7 @@ fr_status fr_solver_set_sgs_mlp(fr_solver* s, const float* host_w);
  * fr_mlp_n_trained() floats).  loss_grad gives the gradient of
  * (1/n) sum sw (c(x) - y)^2 over the trained parameters and the loss; it
  * needs fr_mlp_scratch_floats(n) floats of caller scratch and is
- * deterministic.  adam applies one Adam step (beta 0.9 / 0.999, eps 1e-8;
+ * deterministic: the same bits on every run and every GPU.  adam applies one Adam step (beta 0.9 / 0.999, eps 1e-8;
  * step counts from 1). */
 long long fr_mlp_scratch_floats(long long n);
 fr_status fr_mlp_forward(const float* d_w, const float* d_x, long long n, float* d_out, void* stream);

@@ -46,8 +46,8 @@ def test_batch_instances_equal_their_own_solvers(tune):
         b.autotune(2)
     l0 = b.launch_count()
     b.advance(3, 1e-3)
-    # hex P3 NS: gradient + fused interface/update; hex P2 NS: gradient, interface, update (runs of an odd
-    # number of points); quad P3 Euler: the fused interface/update kernel alone
+    # hex P3 NS: gradient + fused interface/update; hex P2 NS: gradient, interface, update; quad P3 Euler: the
+    # fused interface/update kernel alone
     assert b.launch_count() - l0 == 3 * 5 * (2 + 3 + 1)
     for i in range(len(INSTANCES)):
         assert np.array_equal(b.get_state(i), refs[i]), i

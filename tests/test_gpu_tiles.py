@@ -1,10 +1,9 @@
 """Every compiled tile variant of the gradient and update kernels -- elements
-and threads per block, register budget, and persistent blocks that prefetch
-their next element block -- gives the same state, bit for bit.
+and threads per block, register budget, and persistent blocks that walk over
+element blocks -- gives the same state, bit for bit.
 
 The mesh (12^3 hexes, P = 3) has more element blocks than the B200 keeps
-resident at once, so the persistent variants run several blocks each and
-their prefetch path is exercised."""
+resident at once, so the persistent variants run several blocks each."""
 import numpy as np
 import pytest
 
