@@ -5,6 +5,7 @@
 #include <string>
 
 #include "fr_batch_merged.cuh"
+#include "fr_launch.hpp"
 
 namespace frb {
 
@@ -84,14 +85,9 @@ fr_status launch_t(const void* grads, const void* faces, bool any_face, const vo
   const auto& U = *static_cast<const MergedUpds<TC>*>(upds);
   constexpr size_t smg = std::max({merged_grad_smem<2, TC>(), merged_grad_smem<3, TC>(), merged_grad_smem<4, TC>()});
   constexpr size_t smu = std::max({merged_upd_smem<2, TC>(), merged_upd_smem<3, TC>(), merged_upd_smem<4, TC>()});
-  static bool once = [] {
-    cudaFuncSetAttribute((const void*)fr_merged_grad_kernel<TC, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smg);
-    cudaFuncSetAttribute((const void*)fr_merged_upd_kernel<TC, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smu);
-    return true;
-  }();
-  (void)once;
+  static SmemLimit limit_g, limit_u;
+  limit_g((const void*)fr_merged_grad_kernel<TC, MINB>, smg);
+  limit_u((const void*)fr_merged_upd_kernel<TC, MINB>, smu);
   long long ng = G.s[0].nblk + G.s[1].nblk + G.s[2].nblk;
   long long nu = U.s[0].nblk + U.s[1].nblk + U.s[2].nblk;
   long long nf = Fc.s[0].nblk + Fc.s[1].nblk + Fc.s[2].nblk;

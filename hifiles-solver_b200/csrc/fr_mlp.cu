@@ -19,6 +19,7 @@
 #include <string>
 
 #include "fr_b200.h"
+#include "fr_launch.hpp"
 #include "fr_mlp.cuh"
 
 namespace frb {
@@ -415,9 +416,8 @@ fr_status fr_mlp_loss_grad(const float* w, const float* x, const float* y, const
   if (nblk > 0x7fffffffLL) return mlp_fail(FR_ERR_ARG, "batch too large");
   cudaStream_t st = (cudaStream_t)stream;
   const float inv_n = (float)(1.0 / (double)n);
-  static bool once = (cudaFuncSetAttribute(fr_mlp_loss_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)kGradSmem), true);
-  (void)once;
+  static SmemLimit limit;
+  limit((const void*)fr_mlp_loss_grad_kernel, kGradSmem);
   const int grid = (int)(nblk < kGradCtas ? nblk : kGradCtas);
   fr_mlp_loss_grad_kernel<<<grid, kGradThreads, kGradSmem, st>>>(w, x, y, sw, n, inv_n, scratch);
   fr_mlp_reduce_kernel<<<(kMlpTrain + 1 + 31) / 32, 32 * kRedRows, 0, st>>>(scratch, grid, inv_n, grad, loss);

@@ -10,6 +10,7 @@
 #include "fr_batch_merged.cuh"
 #include "fr_fused.cuh"
 #include "fr_host.hpp"
+#include "fr_launch.hpp"
 #include "fr_tiles.hpp"
 
 namespace frb {
@@ -67,11 +68,6 @@ struct Runner {
     return 0;
   }
 };
-
-static void set_smem(const void* k, size_t bytes)
-{
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
 
 template <int DIM, int P, typename TC>
 struct RunnerT : Runner {
@@ -141,8 +137,8 @@ struct RunnerT : Runner {
       constexpr int PERS = Tiles<DIM, P>::grad[I].pers;
       constexpr size_t sm = grad_smem_bytes<DIM, P, EPB, TC, LES>();
       const void* kfn = (const void*)fr_grad_kernel<DIM, P, EPB, NT, TC, LES, MINB, 1, PERS>;
-      static bool once = (set_smem(kfn, sm), true);
-      (void)once;
+      static SmemLimit limit;
+      limit(kfn, sm);
       long long grid = (E + EPB - 1) / EPB;
       if (PERS) {
         // persistent blocks: as many as are resident at once
@@ -206,8 +202,8 @@ struct RunnerT : Runner {
     constexpr size_t sm = update_smem_bytes<DIM, P, EPB, NT, VISC, MODE, TC>();
     constexpr int FUSED = FU ? 1 : 0;
     const void* kfn = (const void*)fr_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC, FUSED, RS, MB>;
-    static bool once = (set_smem(kfn, sm), true);
-    (void)once;
+    static SmemLimit limit;
+    limit(kfn, sm);
     fr_update_kernel<DIM, P, EPB, NT, VISC, MODE, TC, FUSED, RS, MB><<<(unsigned)((E + EPB - 1) / EPB), NT, sm, s>>>(
         b.U, b.REG, (TC*)b.UF[cur ^ 1], (const TC*)b.UF[cur], (const TC*)b.CF, b.mate, b.side, (const TC*)b.VF,
         (const TC*)b.ND, (const TC*)b.DV, (const TC*)b.JG, (const TC*)b.nL, (const TC*)b.tdA, b.idetj,
