@@ -61,7 +61,7 @@ int diag_epb(int nu)
 // pass; a thread then forms the quantities of one point.  blockIdx.x walks over
 // groups of epb elements, blockIdx.y over the passes.
 template <int D, typename TG, int NQ>
-__global__ void __launch_bounds__(kDiagThreads)
+__global__ void __launch_bounds__(kDiagThreads, 5)
 fr_diag_kernel(const double* __restrict__ U, const TG* __restrict__ G, const double* __restrict__ opp,
                const double* __restrict__ W, const double* __restrict__ detj, long long E, int nu, int nc,
                double gamma, int epb, int ldk, double* __restrict__ partial)
